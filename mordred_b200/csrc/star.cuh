@@ -118,5 +118,7 @@ int launch_list(const mb_star_args* a, cudaStream_t stream, const DeviceState* d
 int list_init_device(const DeviceState& ds);
 // Host: the same for the batched multi-query kernel (batch.cu).
 int batch_init_device(const DeviceState& ds);
+// Host: the same for the planner's kernels (mlp.cu).
+int mlp_init_device(const DeviceState& ds);
 
 }  // namespace mb
