@@ -35,6 +35,7 @@ static int init_device_locked(int dev) {
   int e = star_init_device(ds);
   if (e == MB_OK) e = batch_init_device(ds);
   if (e == MB_OK) e = list_init_device(ds);
+  if (e == MB_OK) e = select_init_device(ds);
   if (e == MB_OK) e = mlp_init_device(ds);
   if (e != MB_OK) return e;
   ds.device = dev;

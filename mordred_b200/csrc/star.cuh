@@ -118,7 +118,8 @@ int launch_list(const mb_star_args* a, cudaStream_t stream, const DeviceState* d
 int list_init_device(const DeviceState& ds);
 // Host: the same for the batched multi-query kernel (batch.cu).
 int batch_init_device(const DeviceState& ds);
-// Host: the same for the planner's kernels (mlp.cu).
+// Host: the same for the selection kernels (compact.cu) and the planner's (mlp.cu).
+int select_init_device(const DeviceState& ds);
 int mlp_init_device(const DeviceState& ds);
 
 }  // namespace mb
