@@ -213,7 +213,7 @@ __device__ __forceinline__ void batch_match(const AQ& A, void* const* s_res, int
   if (A.soff >= 0) {
     const int fam = aq_family(A), j = aq_member(A);
     const int copy = (A.flags >> 5) & 1 ? static_cast<int>(threadIdx.x & (kScalarCopies - 1)) : 0;
-    atomicAdd(reinterpret_cast<unsigned long long*>(smem + A.soff) + g * fam + copy, w);
+    smem_add_i64(reinterpret_cast<unsigned long long*>(smem + A.soff) + g * fam + copy, static_cast<int>(u));
     if (!c4) return;
     // the first row of a group in this CTA writes the group's keys
     uint32_t* s_touch = reinterpret_cast<uint32_t*>(smem + A.soff - 8 * j + 8 * A.total * fam) +

@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(kListThreads) list_kernel(const __grid_constan
         continue;
       }
       if (P.gmode == kGroupSmem) {
-        atomicAdd(&s_sum[h], w);
+        smem_add_i64(&s_sum[h], val);
         const uint32_t bit = 1u << (h & 31);
         if (!(s_touch[h >> 5] & bit) && !(atomicOr(&s_touch[h >> 5], bit) & bit) && P.res_layout != MB_RES_DENSE)
           list_keys(P, h, gv[i]);

@@ -264,7 +264,7 @@ __device__ __forceinline__ void aggregate_rows(const StarPlan& P, const L& ld, u
       continue;
     }
     if (P.gmode == kGroupSmem) {
-      atomicAdd(&s_sum[h], w);
+      smem_add_i64(&s_sum[h], val);
       const uint32_t bit = 1u << (h & 31);
       if (!(s_touch[h >> 5] & bit)) {
         if (!(atomicOr(&s_touch[h >> 5], bit) & bit) && P.res_layout != MB_RES_DENSE)
