@@ -5,24 +5,31 @@
 //     a ring of shared-memory stages with 1-D bulk copies (cp.async.bulk, no multicast);
 //   * per row, each needed dimension is looked up once in its packed attribute table (PAT,
 //     one 32-bit word per hash slot: bit 31 present, attribute fields below) and the word
-//     replaces the key in the stage;
-//   * predicates are evaluated for all queries at once: for every attribute some query
-//     constrains, a table built per batch maps each value of the queries' range hull to
-//     the bitmask of queries accepting it (queries that do not constrain the attribute
+//     replaces the key in the stage; in small batches only while some query left for the row
+//     reads that dimension;
+//   * predicates are evaluated for all queries at once: tables built per batch map an
+//     attribute's value — or the values of several attributes with small domains together —
+//     to the bitmask of queries accepting it (queries that do not constrain an attribute
 //     accept every value), and a table over the 16 dimension-presence patterns does the
-//     same for the dimensions each query needs; a row ANDs one mask per attribute and
-//     visits only the queries left set;
-//   * the (row, query) pairs a warp finds go to a list in shared memory; a full list is
-//     aggregated 32 pairs at a time, one per lane, by branch-light code driven by a
-//     32-byte per-query descriptor: the pair's 64-bit value is added to the query's
-//     scalar or shared-memory group array (flushed once per CTA) or its group array in L2.
+//     same for the dimensions each query needs; a row ANDs one mask per table and visits
+//     only the queries left set;
+//   * queries that add the same expression to the same group index form a class (the forms
+//     of one template). Class by class, the (row, query) pairs a warp finds go to a list in
+//     shared memory and are aggregated 32 pairs at a time, one per lane: value, keys and
+//     group come from fields that are the same for all lanes, the destination from a
+//     16-byte record of the query — its scalar or shared-memory group array (flushed once
+//     per CTA) or its group array in L2. Queries beyond the four largest classes are
+//     aggregated from a 32-byte descriptor of their own.
 // A query's result equals its lone run through mb_star_query with filtered hash tables:
 // with unique dimension keys, "the key is in the filtered table" is "the row's
 // attributes pass the filter", and the payload is the attribute itself; sums are
 // integers, so the order of additions cannot change a bit.
 #include <algorithm>
+#include <climits>
+#include <cstddef>
 #include <cstring>
 #include <mutex>
+#include <vector>
 
 #include "common.cuh"
 
@@ -33,7 +40,10 @@ constexpr int kBatchStages = 8;
 constexpr int kMaxPredFields = 8;
 constexpr int kMaskWordsMax = MB_BATCH_MAX_QUERIES / 32;
 constexpr int kSmemTableMaxEntries = 512;  // predicate tables up to this many values sit in shared memory
-constexpr int kMatchListMax = 1024;        // (row, query) pairs a consumer warp collects before aggregating
+constexpr int kCombineMaxEntries = 320;    // entries of a table that combines several small attributes
+constexpr int kMaxComponents = 4;          // attributes a table combines
+constexpr int kMaxClasses = 4;
+constexpr int kMatchListCap = 512;         // pairs of one class a consumer warp collects before aggregating
 constexpr int kColPad = 4;                 // words between staged columns: the same row of two columns
                                            // falls in different banks (and stays 16-byte aligned)
 constexpr int kMaxStageCols = MB_NUM_FACT_COLS + 1;
@@ -72,6 +82,17 @@ __device__ __forceinline__ int aq_family(const AQ& A) { return (A.flags >> 8) & 
 __device__ __forceinline__ int aq_member(const AQ& A) { return (A.flags >> 17) & 0x1ff; }
 static_assert(sizeof(AQ) == 32, "aggregation descriptor size");
 
+// What a match of a query needs when its class supplies value, group and keys (16 bytes,
+// shared memory).
+struct __align__(16) QD {
+  int soff;    // shared-memory byte offset of the sums; < 0: at s_addr[query]
+  int stride;  // bytes between the sums of neighbouring groups
+  int touch;   // >= 0: shared-memory byte offset of the key touch bitmap; -1: no keys to
+               // write; -2: written on every match
+  int pad;
+};
+static_assert(sizeof(QD) == 16, "match record size");
+
 // Per-query descriptor in the launch parameters (96 bytes).
 struct BQ {
   AQ a;
@@ -83,6 +104,51 @@ struct BQ {
 };
 static_assert(sizeof(BQ) == 96, "descriptor size");
 
+// A field of a staged row: word offset of its column in the stage, shift, mask.
+struct Field {
+  int word, shift;
+  unsigned mask;
+};
+
+// An attribute the batch constrains, and its part in a table of query masks. A table covers
+// one attribute or several with few values, and holds one mask per combination of their
+// indexes (the sum of index * mul). An attribute's index is its value less `min`, or its
+// interval when interval-coded, or one more than the last of these for every value outside
+// the queries' hull (which no query constraining the attribute accepts).
+// Interval coding of a wide attribute (hull wider than kSmemTableMaxEntries values): the
+// queries' range end points cut the hull into nint intervals on which every query's verdict
+// is constant; the table holds one mask per interval. A value v (relative to min) is in
+// interval i when bp[i] <= v < bp[i+1]; bucket v >> bkt_shift of a shared-memory index gives
+// the interval of the bucket's first value, and a short forward scan over the end points
+// finishes the search.
+struct Attr {
+  Field f;
+  int code, scode;         // row-schema and stage field codes
+  int min, n;              // hull
+  int nint, bp_off, bkt_shift;
+  int bps_off, bkt_off;    // shared-memory byte offsets of end points and bucket index
+  int mul;
+  int last;                // 1: the last attribute of its table, which the fields below describe
+  int ent, smem_off;       // entries; byte offset in shared memory, -1: in the workspace
+  long long goff;          // word offset in the workspace
+};
+
+// A dimension the batch reads: where its key and its word lie in the stage, its table, and
+// per query whether the row must exist (need) and whether the query reads the word at all.
+struct Dim {
+  int d, key_word, word;
+  int slots, kmin;
+  const unsigned* pat;
+  unsigned need[kMaskWordsMax], use[kMaskWordsMax];
+};
+
+// What the queries of a class share (see AQ).
+struct Class {
+  Field a0, a1, k0, k1;
+  unsigned kmul0, kmul1, bias;
+  int total, op, scalar, two_keys;
+};
+
 struct BatchPlan {
   long long n, nfull;
   int ncols;                       // staged fact columns
@@ -90,31 +156,22 @@ struct BatchPlan {
   int cidx[13];                    // row-schema column -> stage column (-1: absent)
   int stage_dim[kMaxStageCols];    // stage column -> dimension whose word it holds (-1: fact column)
   int ndims;
-  int dim_list[4];
-  int key_stage[4];
-  const unsigned* pat[4];
-  int pat_slots[4], pat_kmin[4];
+  Dim dim[4];
   int nq, nwords;
-  int nfields;                     // attributes some query constrains
-  int f_code[kMaxPredFields], f_scode[kMaxPredFields], f_min[kMaxPredFields], f_n[kMaxPredFields];
-  int f_smem_off[kMaxPredFields];  // byte offset of the table in shared memory, -1: workspace
-  long long f_goff[kMaxPredFields];// word offset of the table in the workspace
-  int f_ent[kMaxPredFields];       // table entries: f_n, or f_nint for an interval-coded attribute
-  // Interval coding of a wide attribute (hull wider than kSmemTableMaxEntries values): the
-  // queries' range end points cut the hull into f_nint intervals on which every query's
-  // verdict is constant; the table holds one mask per interval. A value v (relative to
-  // f_min) is in interval i when bp[i] <= v < bp[i+1]; bucket v >> f_shift of a shared-
-  // memory index gives the interval of the bucket's first value, and a short forward
-  // scan over the end points finishes the search.
-  int f_nint[kMaxPredFields], f_bp_off[kMaxPredFields], f_shift[kMaxPredFields];
-  int f_bps_off[kMaxPredFields], f_bkt_off[kMaxPredFields];  // shared-memory byte offsets
+  // The attributes some query constrains: those of fact columns first (nfact), then those of
+  // dimension words; attributes that share a table are neighbours.
+  int nfields, nfact;
+  Attr at[kMaxPredFields];
   int bp[kMaxBreakpoints];
-  unsigned outside[kMaxPredFields][kMaskWordsMax];  // mask for values outside the hull
   unsigned pres_mask[16][kMaskWordsMax];
+  unsigned all[kMaskWordsMax];
+  int ncls, others;                // classes; 1: some queries belong to none
+  Class cls[kMaxClasses];
+  unsigned cls_mask[kMaxClasses + 1][kMaskWordsMax];  // ... the last: queries without a class
   unsigned* tables;                // workspace
   long long table_entries;
-  int stages, stage_words, list_cap;
-  int smem_acc_off, smem_aq_off, smem_res_off, smem_pres_off, smem_out_off, smem_list_off;
+  int stages, stage_words;
+  int smem_acc_off, smem_aq_off, smem_qd_off, smem_res_off, smem_addr_off, smem_pres_off, smem_list_off;
   int acc_words;                   // 8-byte scalar words (kScalarCopies per scalar query)
   int smem_groups_off, smem_groups_words, smem_stage_off;
   unsigned int* status;
@@ -126,11 +183,11 @@ struct BatchPlan {
 };
 static_assert(sizeof(BatchPlan) < 32000, "launch parameter limit");
 
+// (key - kmin) % slots: keys within two table lengths of kmin without a division.
 __device__ __forceinline__ int bslot(int key, int slots, int kmin) {
-  const int d = static_cast<int>(static_cast<unsigned>(key) - static_cast<unsigned>(kmin));
-  if (static_cast<unsigned>(d) < static_cast<unsigned>(slots)) return d;
-  if (static_cast<unsigned>(d) < 2u * static_cast<unsigned>(slots)) return d - slots;
-  return d % slots;
+  const unsigned d = static_cast<unsigned>(key) - static_cast<unsigned>(kmin), n = static_cast<unsigned>(slots);
+  const unsigned h = min(d, d - n);
+  return h < n ? static_cast<int>(h) : slow_mod(static_cast<int>(d), slots);
 }
 
 // Physical tile of scan position t (CTA b takes positions b, b + G, b + 2G, ...). The
@@ -241,44 +298,67 @@ __device__ __forceinline__ void batch_match(const AQ& A, void* const* s_res, int
     res[4 * g] = k0;
 }
 
-// The queries accepting one row: presence mask AND one mask per constrained attribute.
-// `get(code)` reads a field of the row.
-template <int NWM, class Get>
-__device__ __forceinline__ void batch_row_mask(const BatchPlan& P, unsigned pres, Get get, const unsigned* s_pres,
-                                               const unsigned* s_out, const unsigned char* smem, unsigned (&m)[NWM]) {
+__device__ __forceinline__ int field_of(const int* row, const Field& f) {
+  return static_cast<int>((static_cast<unsigned>(row[f.word]) >> f.shift) & f.mask);
+}
+
+// Index of a value among attribute A's table indexes (see Attr).
+__device__ __forceinline__ int attr_index(const BatchPlan& P, const Attr& A, int value, const unsigned char* smem) {
+  const unsigned v = static_cast<unsigned>(value) - static_cast<unsigned>(A.min);
+  const unsigned n = static_cast<unsigned>(A.n);
+  if (A.nint == 0) return static_cast<int>(min(v, n));
+  if (v >= n) return A.nint;
+  const int* bp = reinterpret_cast<const int*>(smem + A.bps_off);
+  int e = reinterpret_cast<const uint16_t*>(smem + A.bkt_off)[v >> A.bkt_shift];
+  while (e + 1 < A.nint && bp[e + 1] <= static_cast<int>(v)) ++e;
+  return e;
+}
+
+// m &= entry e of the table that attribute A closes. Entries of eight words lie in two arrays
+// of four, so that the 16-byte loads of neighbouring entries fall in different banks.
+template <int NWM>
+__device__ __forceinline__ void and_entry(const BatchPlan& P, const Attr& A, int e, const unsigned char* smem,
+                                          unsigned (&m)[NWM]) {
+  const unsigned* base = A.smem_off >= 0 ? reinterpret_cast<const unsigned*>(smem + A.smem_off) : P.tables + A.goff;
+  if constexpr (NWM >= 4) {
 #pragma unroll
-  for (int w = 0; w < NWM; ++w) m[w] = s_pres[pres * kMaskWordsMax + w];
+    for (int h = 0; h < NWM / 4; ++h) {
+      const uint4 u = *reinterpret_cast<const uint4*>(base + 4 * (h * A.ent + e));
+      m[4 * h] &= u.x;
+      m[4 * h + 1] &= u.y;
+      m[4 * h + 2] &= u.z;
+      m[4 * h + 3] &= u.w;
+    }
+  } else if constexpr (NWM == 2) {
+    const uint2 u = *reinterpret_cast<const uint2*>(base + 2 * e);
+    m[0] &= u.x;
+    m[1] &= u.y;
+  } else {
+    m[0] &= base[e];
+  }
+}
+
+// The masks of GR rows (row r at stage pointer row + 32 r) ANDed with the tables over fact
+// columns (DIMS false) or over dimension words.
+template <int NWM, int GR, bool DIMS>
+__device__ __forceinline__ void and_tables(const BatchPlan& P, const int* row, const unsigned char* smem,
+                                           unsigned (&m)[GR][NWM]) {
+  int e[GR];
 #pragma unroll
-  for (int f = 0; f < kMaxPredFields; ++f) {
-    if (f >= P.nfields) break;
-    // with one mask word an empty mask ends the row early; with more, rows nearly always
-    // keep some query and the test would cost more than it saves
-    if (NWM == 1 && m[0] == 0) return;
-    const int v = get(P.f_scode[f]) - P.f_min[f];
-    const unsigned* t;
-    if (static_cast<unsigned>(v) < static_cast<unsigned>(P.f_n[f])) {
-      int e = v;
-      if (P.f_nint[f] > 0) {
-        const int* bp = reinterpret_cast<const int*>(smem + P.f_bps_off[f]);
-        e = reinterpret_cast<const uint16_t*>(smem + P.f_bkt_off[f])[v >> P.f_shift[f]];
-        while (e + 1 < P.f_nint[f] && bp[e + 1] <= v) ++e;
+  for (int r = 0; r < GR; ++r) e[r] = 0;
+#pragma unroll
+  for (int i = 0; i < kMaxPredFields; ++i) {
+    if (i >= (DIMS ? P.nfields : P.nfact)) break;
+    if (DIMS && i < P.nfact) continue;
+    const Attr& A = P.at[i];
+#pragma unroll
+    for (int r = 0; r < GR; ++r) e[r] += attr_index(P, A, field_of(row + 32 * r, A.f), smem) * A.mul;
+    if (A.last) {
+#pragma unroll
+      for (int r = 0; r < GR; ++r) {
+        and_entry<NWM>(P, A, e[r], smem, m[r]);
+        e[r] = 0;
       }
-      t = P.f_smem_off[f] >= 0 ? reinterpret_cast<const unsigned*>(smem + P.f_smem_off[f]) + e * P.nwords
-                               : P.tables + P.f_goff[f] + static_cast<long long>(e) * P.nwords;
-    } else
-      t = s_out + f * kMaskWordsMax;
-    if (NWM >= 4) {
-#pragma unroll
-      for (int w = 0; w < NWM; w += 4) {
-        const uint4 u = *reinterpret_cast<const uint4*>(t + w);
-        m[w] &= u.x;
-        m[w + 1] &= u.y;
-        m[w + 2] &= u.z;
-        m[w + 3] &= u.w;
-      }
-    } else {
-#pragma unroll
-      for (int w = 0; w < NWM; ++w) m[w] &= t[w];
     }
   }
 }
@@ -289,13 +369,21 @@ __global__ void __launch_bounds__((NCW + 1) * 32, 1) batch_kernel(const __grid_c
   constexpr int TILE = NCW * WROWS;
   constexpr int CS = TILE + kColPad;  // stage column stride (words)
   constexpr int NWARPS = NCW + 1;
+  // rows a lane works on at a time: their table lookups are in flight together and their
+  // matches share the aggregation passes (as many as eight mask words in registers allow)
+  constexpr int GR = ITEMS * NWM <= 8 ? ITEMS : NWM >= 8 ? 1 : 8 / NWM;
+  static_assert(ITEMS % GR == 0, "whole groups of rows");
+  // with one or two mask words a row often runs out of queries on its fact columns: it then
+  // looks up a dimension only if a query that reads it is left
+  constexpr bool LAZY = NWM <= 2;
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);
   uint64_t* empty = full + kBatchStages;
   AQ* s_aq = reinterpret_cast<AQ*>(smem + P.smem_aq_off);
+  QD* s_qd = reinterpret_cast<QD*>(smem + P.smem_qd_off);
   void** s_res = reinterpret_cast<void**>(smem + P.smem_res_off);
+  unsigned char** s_addr = reinterpret_cast<unsigned char**>(smem + P.smem_addr_off);
   unsigned* s_pres = reinterpret_cast<unsigned*>(smem + P.smem_pres_off);
-  unsigned* s_out = reinterpret_cast<unsigned*>(smem + P.smem_out_off);
   int* stage_base = reinterpret_cast<int*>(smem + P.smem_stage_off);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int S = P.stages;
@@ -304,22 +392,37 @@ __global__ void __launch_bounds__((NCW + 1) * 32, 1) batch_kernel(const __grid_c
   {
     unsigned long long* s_acc = reinterpret_cast<unsigned long long*>(smem + P.smem_acc_off);
     for (int w = tid; w < P.acc_words; w += NWARPS * 32) s_acc[w] = 0;
-    for (int q = tid; q < P.nq; q += NWARPS * 32) s_res[q] = P.q[q].res;
-    unsigned* dst = reinterpret_cast<unsigned*>(s_aq);
-    for (int w = tid; w < P.nq * 8; w += NWARPS * 32) dst[w] = reinterpret_cast<const unsigned*>(&P.q[w >> 3].a)[w & 7];
+    for (int q = tid; q < P.nq; q += NWARPS * 32) {
+      const BQ& Q = P.q[q];
+      const AQ A = Q.a;
+      const bool c4 = (A.flags >> 2) & 1;
+      const int nk = (A.flags >> 3) & 3;
+      s_aq[q] = A;
+      s_res[q] = Q.res;
+      s_addr[q] = static_cast<unsigned char*>(Q.res) + (c4 ? 8 : 0);
+      QD d;
+      d.soff = A.soff >= 0 ? A.soff : -1;
+      d.stride = A.soff < 0 ? (c4 ? 16 : 8) : (A.flags >> 5) & 1 ? 8 : 8 * aq_family(A);
+      d.touch = !c4 || nk == 0 ? -1
+                : A.soff >= 0  ? A.soff - 8 * aq_member(A) + 8 * A.total * aq_family(A) +
+                                    4 * ((A.total + 31) >> 5) * aq_member(A)
+                : A.soff <= -2 ? -A.soff - 2
+                               : -2;
+      d.pad = 0;
+      s_qd[q] = d;
+    }
     for (int w = tid; w < 16 * kMaskWordsMax; w += NWARPS * 32) s_pres[w] = (&P.pres_mask[0][0])[w];
-    for (int w = tid; w < kMaxPredFields * kMaskWordsMax; w += NWARPS * 32) s_out[w] = (&P.outside[0][0])[w];
     unsigned* g = reinterpret_cast<unsigned*>(smem + P.smem_groups_off);
     for (int w = tid; w < P.smem_groups_words; w += NWARPS * 32) g[w] = 0;
     for (int f = 0; f < P.nfields; ++f) {
-      if (P.f_smem_off[f] < 0) continue;
-      unsigned* t = reinterpret_cast<unsigned*>(smem + P.f_smem_off[f]);
-      const unsigned* s = P.tables + P.f_goff[f];
-      for (int w = tid; w < P.f_ent[f] * P.nwords; w += NWARPS * 32) t[w] = s[w];
-      if (P.f_nint[f] > 0) {
-        int* bp = reinterpret_cast<int*>(smem + P.f_bps_off[f]);
-        for (int i = tid; i < P.f_nint[f]; i += NWARPS * 32) bp[i] = P.bp[P.f_bp_off[f] + i];
+      const Attr& A = P.at[f];
+      if (A.last && A.smem_off >= 0) {
+        unsigned* dst = reinterpret_cast<unsigned*>(smem + A.smem_off);
+        const unsigned* src = P.tables + A.goff;
+        for (int w = tid; w < A.ent * NWM; w += NWARPS * 32) dst[w] = src[w];
       }
+      int* bp = reinterpret_cast<int*>(smem + A.bps_off);
+      for (int i = tid; i < A.nint; i += NWARPS * 32) bp[i] = P.bp[A.bp_off + i];
     }
   }
   if (tid == 0) {
@@ -332,13 +435,14 @@ __global__ void __launch_bounds__((NCW + 1) * 32, 1) batch_kernel(const __grid_c
   __syncthreads();
   // bucket indexes of the interval-coded attributes: the interval of each bucket's first value
   for (int f = 0; f < P.nfields; ++f) {
-    if (P.f_nint[f] == 0) continue;
-    const int* bp = reinterpret_cast<const int*>(smem + P.f_bps_off[f]);
-    uint16_t* bkt = reinterpret_cast<uint16_t*>(smem + P.f_bkt_off[f]);
-    const int nb = ((P.f_n[f] - 1) >> P.f_shift[f]) + 1;
+    const Attr& A = P.at[f];
+    if (A.nint == 0) continue;
+    const int* bp = reinterpret_cast<const int*>(smem + A.bps_off);
+    uint16_t* bkt = reinterpret_cast<uint16_t*>(smem + A.bkt_off);
+    const int nb = ((A.n - 1) >> A.bkt_shift) + 1;
     for (int b = tid; b < nb; b += NWARPS * 32) {
-      const int v0 = b << P.f_shift[f];
-      int lo = 0, hi = P.f_nint[f] - 1;  // bp[0] = 0 <= v0: find the last bp[i] <= v0
+      const int v0 = b << A.bkt_shift;
+      int lo = 0, hi = A.nint - 1;  // bp[0] = 0 <= v0: find the last bp[i] <= v0
       while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (bp[mid] <= v0)
@@ -405,7 +509,7 @@ __global__ void __launch_bounds__((NCW + 1) * 32, 1) batch_kernel(const __grid_c
     }
   } else {
     const int cw = warp - 1;
-    unsigned* mlist = reinterpret_cast<unsigned*>(smem + P.smem_list_off) + cw * P.list_cap;
+    uint16_t* mlist = reinterpret_cast<uint16_t*>(smem + P.smem_list_off) + cw * kMatchListCap;
     int s = 0;
     uint32_t phase = 0;
     for (long long k = 0; k < my_tiles; ++k) {
@@ -415,117 +519,187 @@ __global__ void __launch_bounds__((NCW + 1) * 32, 1) batch_kernel(const __grid_c
         break;
       }
       int* wst = stage_base + s * P.stage_words + cw * WROWS;
-      // ---- dimension words, once per row for the whole batch -------------------
-      for (int t = 0; t < P.ndims; ++t) {
-        const int d = P.dim_list[t];
-        const int* kcol = wst + P.key_stage[d] * CS;
-        int* out = wst + P.cidx[MB_COL_DIM_S + d] * CS;
-        const unsigned* pat = P.pat[d];
-        const int slots = P.pat_slots[d], kmin = P.pat_kmin[d];
-        unsigned wv[ITEMS];
-        auto lookup = [&](int key) -> unsigned {
-          const int h = bslot(key, slots, kmin);
-          if (h < 0) {
-            bad_probe = true;
-            return 0u;
+#pragma unroll 1
+      for (int i0 = 0; i0 < ITEMS; i0 += GR) {
+        // ---- the queries accepting each row (lane l has rows i0 * 32 + l, + 32, ...) ----
+        int* row = wst + i0 * 32 + lane;
+        unsigned m[GR][NWM];
+#pragma unroll
+        for (int r = 0; r < GR; ++r)
+#pragma unroll
+          for (int w = 0; w < NWM; ++w) m[r][w] = P.all[w];
+        auto look_up = [&](unsigned (&word)[GR][4]) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+#pragma unroll
+            for (int r = 0; r < GR; ++r) word[r][j] = 0;
+            if (j >= P.ndims) continue;
+            const Dim& D = P.dim[j];
+#pragma unroll
+            for (int r = 0; r < GR; ++r) {
+              const int h = bslot(row[32 * r + D.key_word], D.slots, D.kmin);
+              bool want = true;
+              if constexpr (LAZY) {
+                want = false;
+#pragma unroll
+                for (int w = 0; w < NWM; ++w) want = want || (m[r][w] & D.use[w]) != 0;
+              }
+              if (h < 0)
+                bad_probe = true;
+              else if (want)
+                word[r][j] = __ldg(D.pat + h);
+            }
           }
-          return __ldg(pat + h);
         };
-        if constexpr (ITEMS % 4 == 0) {
+        auto keep_words = [&](const unsigned (&word)[GR][4]) {
 #pragma unroll
-          for (int j = 0; j < ITEMS / 4; ++j) {
-            const int4 kv = lds128(kcol + (j * 32 + lane) * 4);
-            wv[4 * j] = lookup(kv.x);
-            wv[4 * j + 1] = lookup(kv.y);
-            wv[4 * j + 2] = lookup(kv.z);
-            wv[4 * j + 3] = lookup(kv.w);
+          for (int j = 0; j < 4; ++j) {
+            if (j >= P.ndims) break;
+#pragma unroll
+            for (int r = 0; r < GR; ++r) row[32 * r + P.dim[j].word] = static_cast<int>(word[r][j]);
           }
+        };
+        if constexpr (LAZY) {
+          and_tables<NWM, GR, false>(P, row, smem, m);
+          unsigned word[GR][4];
+          look_up(word);
+          keep_words(word);
 #pragma unroll
-          for (int j = 0; j < ITEMS / 4; ++j) {
-            int4 o;
-            o.x = static_cast<int>(wv[4 * j]);
-            o.y = static_cast<int>(wv[4 * j + 1]);
-            o.z = static_cast<int>(wv[4 * j + 2]);
-            o.w = static_cast<int>(wv[4 * j + 3]);
-            *reinterpret_cast<int4*>(out + (j * 32 + lane) * 4) = o;
+          for (int j = 0; j < 4; ++j) {
+            if (j >= P.ndims) break;
+#pragma unroll
+            for (int r = 0; r < GR; ++r)
+#pragma unroll
+              for (int w = 0; w < NWM; ++w) m[r][w] &= word[r][j] >> 31 ? kFullMask : ~P.dim[j].need[w];
           }
         } else {
+          unsigned word[GR][4];
+          look_up(word);
+          and_tables<NWM, GR, false>(P, row, smem, m);  // while the words are on their way
+          keep_words(word);
 #pragma unroll
-          for (int e = 0; e < ITEMS; ++e) wv[e] = lookup(kcol[e * 32 + lane]);
+          for (int r = 0; r < GR; ++r) {
+            unsigned pres = 0;
 #pragma unroll
-          for (int e = 0; e < ITEMS; ++e) out[e * 32 + lane] = static_cast<int>(wv[e]);
-        }
-      }
-      __syncwarp();
-      // ---- query masks row by row (lane l takes rows l, 32 + l, ...); matches go
-      // through the warp's list so that every lane aggregates one pair at a time ------
-      int lpos = 0;
-      auto flush = [&](int n) {
-        for (int base = 0; base < n; base += 32) {
-          const int idx = base + lane;
-          if (idx < n) {
-            const unsigned pr = mlist[idx];
-            const int row = static_cast<int>(pr >> 16), qi = static_cast<int>(pr & 0xffffu);
-            auto get = [&](int code) { return field_value(wst[(code >> 11) * CS + row], code); };
-            batch_match(load_aq(s_aq, qi), s_res, qi, get, smem, bad_group);
+            for (int j = 0; j < 4; ++j)
+              if (j < P.ndims) pres |= (word[r][j] >> 31) << P.dim[j].d;
+#pragma unroll
+            for (int q = 0; q < NWM; q += 4) {
+              const uint4 u = *reinterpret_cast<const uint4*>(s_pres + pres * kMaskWordsMax + q);
+              m[r][q] &= u.x;
+              m[r][q + 1] &= u.y;
+              m[r][q + 2] &= u.z;
+              m[r][q + 3] &= u.w;
+            }
           }
         }
-        __syncwarp();
-      };
+        and_tables<NWM, GR, true>(P, row, smem, m);
+        // ---- class by class: list the matches, aggregate them (one copy of the code for all
+        // classes: unrolled over them it no longer fits the instruction cache) ----
 #pragma unroll 1
-      for (int i = 0; i < ITEMS; ++i) {
-        const int row = i * 32 + lane;
-        unsigned pres = 0;
-        for (int t = 0; t < P.ndims; ++t) {
-          const int d = P.dim_list[t];
-          pres |= (static_cast<unsigned>(wst[P.cidx[MB_COL_DIM_S + d] * CS + row]) >> 31) << d;
-        }
-        auto get = [&](int code) { return field_value(wst[(code >> 11) * CS + row], code); };
-        unsigned m[NWM];
-        batch_row_mask<NWM>(P, pres, get, s_pres, s_out, smem, m);
-        int cnt = 0;
-#pragma unroll
-        for (int w = 0; w < NWM; ++w) cnt += __popc(m[w]);
-        int incl = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int y = __shfl_up_sync(kFullMask, incl, o);
-          if (lane >= o) incl += y;
-        }
-        const int total = __shfl_sync(kFullMask, incl, 31);
-        if (total == 0) continue;
-        if (lpos + total > P.list_cap) {
-          flush(lpos);
-          lpos = 0;
-        }
-        if (total > P.list_cap) {
-          // more matches than the list holds: this row runs lane by lane
+        for (int c = 0; c <= kMaxClasses; ++c) {
+          if (c < kMaxClasses ? c >= P.ncls : !P.others) continue;
+          int mine = 0;
 #pragma unroll
           for (int w = 0; w < NWM; ++w) {
-            unsigned bits = m[w];
-            while (bits) {
-              const int qi = w * 32 + __ffs(bits) - 1;
-              bits &= bits - 1;
-              batch_match(load_aq(s_aq, qi), s_res, qi, get, smem, bad_group);
+            const unsigned of = P.cls_mask[c][w];
+#pragma unroll
+            for (int r = 0; r < GR; ++r) mine += __popc(m[r][w] & of);
+          }
+          if (!__any_sync(kFullMask, mine != 0)) continue;
+          int up_to = mine;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kFullMask, up_to, o);
+            if (lane >= o) up_to += y;
+          }
+          const int total = __shfl_sync(kFullMask, up_to, 31);
+          if (total > kMatchListCap) {
+            // more matches than the list holds: lane by lane
+#pragma unroll 1
+            for (int k = 0; k < GR * NWM; ++k) {
+              unsigned bits = 0;
+#pragma unroll
+              for (int r = 0; r < GR; ++r)
+#pragma unroll
+                for (int w = 0; w < NWM; ++w)
+                  if (k == r * NWM + w) bits = m[r][w] & P.cls_mask[c][w];
+              const int* mrow = row + 32 * (k / NWM);
+              auto get = [&](int code) { return field_value(mrow[(code >> 11) * CS], code); };
+              while (bits) {
+                const int qi = (k % NWM) * 32 + __ffs(bits) - 1;
+                bits &= bits - 1;
+                batch_match(load_aq(s_aq, qi), s_res, qi, get, smem, bad_group);
+              }
+            }
+            __syncwarp();
+            continue;
+          }
+          uint16_t* at = mlist + (up_to - mine);
+#pragma unroll
+          for (int w = 0; w < NWM; ++w) {
+            const unsigned of = P.cls_mask[c][w];
+            if (of == 0) continue;
+#pragma unroll
+            for (int r = 0; r < GR; ++r) {
+              unsigned bits = m[r][w] & of;
+              while (bits) {
+                const int qi = w * 32 + __ffs(bits) - 1;
+                bits &= bits - 1;
+                *at++ = static_cast<uint16_t>((((i0 + r) * 32 + lane) << 8) | qi);
+              }
             }
           }
           __syncwarp();
-          continue;
-        }
-        int p = lpos + incl - cnt;
-#pragma unroll
-        for (int w = 0; w < NWM; ++w) {
-          unsigned bits = m[w];
-          while (bits) {
-            const int qi = w * 32 + __ffs(bits) - 1;
-            bits &= bits - 1;
-            mlist[p++] = (static_cast<unsigned>(row) << 16) | static_cast<unsigned>(qi);
+          for (int base = 0; base < total; base += 32) {
+            if (base + lane >= total) continue;
+            const unsigned pair = mlist[base + lane];
+            const int qi = static_cast<int>(pair & 255u);
+            const int* mrow = wst + (pair >> 8);
+            if (c == kMaxClasses) {
+              auto get = [&](int code) { return field_value(mrow[(code >> 11) * CS], code); };
+              batch_match(load_aq(s_aq, qi), s_res, qi, get, smem, bad_group);
+              continue;
+            }
+            const Class& C = P.cls[c < kMaxClasses ? c : 0];
+            const unsigned v0 = static_cast<unsigned>(field_of(mrow, C.a0)), v1 = static_cast<unsigned>(field_of(mrow, C.a1));
+            const int v = static_cast<int>(C.op == MB_AGG_SUM ? v0 : C.op == MB_AGG_SUB ? v0 - v1 : v0 * v1);
+            const QD D = s_qd[qi];
+            if (C.scalar) {
+              smem_add_i64(reinterpret_cast<unsigned long long*>(smem + D.soff) + (lane & (kScalarCopies - 1)), v);
+              continue;
+            }
+            const int k0 = field_of(mrow, C.k0), k1 = field_of(mrow, C.k1);
+            const unsigned hh = static_cast<unsigned>(k0) * C.kmul0 + static_cast<unsigned>(k1) * C.kmul1 + C.bias;
+            int g = static_cast<int>(hh);
+            if (hh >= static_cast<unsigned>(C.total)) {
+              g = slow_mod(g, C.total);
+              if (g < 0) {
+                bad_group = true;
+                continue;
+              }
+            }
+            if (D.soff >= 0)
+              smem_add_i64(reinterpret_cast<unsigned long long*>(smem + D.soff + g * D.stride), v);
+            else
+              atomicAdd(reinterpret_cast<unsigned long long*>(s_addr[qi] + static_cast<long long>(g) * D.stride),
+                        static_cast<unsigned long long>(static_cast<long long>(v)));
+            if (D.touch == -1) continue;
+            if (D.touch >= 0) {
+              // the first row of a group in this CTA writes the group's keys
+              uint32_t* touch = reinterpret_cast<uint32_t*>(smem + D.touch) + (g >> 5);
+              const uint32_t bit = 1u << (g & 31);
+              if ((*touch & bit) || (atomicOr(touch, bit) & bit)) continue;
+            }
+            int* out = static_cast<int*>(s_res[qi]) + 4ll * g;
+            if (C.two_keys)
+              *reinterpret_cast<int2*>(out) = make_int2(k0, k1);  // one 8-byte store (16-byte records)
+            else
+              *out = k0;
           }
+          __syncwarp();
         }
-        lpos += total;
-        __syncwarp();
       }
-      flush(lpos);
       __syncwarp();
       if (lane == 0) bmbar_arrive(&empty[s]);
       if (++s == S) {
@@ -538,14 +712,14 @@ __global__ void __launch_bounds__((NCW + 1) * 32, 1) batch_kernel(const __grid_c
       for (long long r = P.nfull * TILE + b * (NCW * 32) + (tid - 32); r < P.n; r += G * (NCW * 32)) {
         int dimw[4] = {0, 0, 0, 0};
         uint32_t pr = 0;
-        for (int t = 0; t < P.ndims; ++t) {
-          const int d = P.dim_list[t];
-          const int h = bslot(batch_load(P, P.key_stage[d], r), P.pat_slots[d], P.pat_kmin[d]);
+        for (int j = 0; j < P.ndims; ++j) {
+          const int d = P.dim[j].d;
+          const int h = bslot(batch_load(P, P.dim[j].key_word / CS, r), P.dim[j].slots, P.dim[j].kmin);
           if (h < 0) {
             bad_probe = true;
             continue;
           }
-          dimw[d] = static_cast<int>(__ldg(P.pat[d] + h));
+          dimw[d] = static_cast<int>(__ldg(P.dim[j].pat + h));
           pr |= (static_cast<unsigned>(dimw[d]) >> 31) << d;
         }
         auto get = [&](int code) {
@@ -554,7 +728,17 @@ __global__ void __launch_bounds__((NCW + 1) * 32, 1) batch_kernel(const __grid_c
           return field_value(d >= 0 ? dimw[d] : batch_load(P, c, r), code);
         };
         unsigned m[NWM];
-        batch_row_mask<NWM>(P, pr, get, s_pres, s_out, smem, m);
+#pragma unroll
+        for (int w = 0; w < NWM; ++w) m[w] = s_pres[pr * kMaskWordsMax + w];
+        int e = 0;
+        for (int f = 0; f < P.nfields; ++f) {
+          const Attr& A = P.at[f];
+          e += attr_index(P, A, get(A.scode), smem) * A.mul;
+          if (A.last) {
+            and_entry<NWM>(P, A, e, smem, m);
+            e = 0;
+          }
+        }
 #pragma unroll
         for (int w = 0; w < NWM; ++w) {
           unsigned bits = m[w];
@@ -593,30 +777,78 @@ __global__ void __launch_bounds__((NCW + 1) * 32, 1) batch_kernel(const __grid_c
   }
 }
 
-// Per-batch query masks: entry (field f, value v), word w holds bit (q - 32w) for every
-// query q that accepts f = f_min + v (every one of its predicates on f holds, or it has none).
-__global__ void batch_mask_kernel(const __grid_constant__ BatchPlan P) {
-  const long long total = P.table_entries * P.nwords;
-  for (long long e = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; e < total;
-       e += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int w = static_cast<int>(e % P.nwords);
-    long long v = e / P.nwords;
-    int f = 0;
-    while (f < P.nfields - 1 && v >= P.f_ent[f]) v -= P.f_ent[f++];
-    // an interval's verdicts are those of its first value
-    const int x = P.f_min[f] + (P.f_nint[f] > 0 ? P.bp[P.f_bp_off[f] + v] : static_cast<int>(v));
-    const int code = P.f_code[f];
+// The tables' entries. Entry e of a table, word w holds bit (q - 32w) for every query q that
+// accepts the entry's values: every one of its predicates on the table's attributes holds
+// there (no value outside an attribute's hull passes a predicate on it). A warp takes 32
+// entries of one table and one word: lane l knows the values of the l-th entry and the ranges
+// of the l-th query, and entry by entry the values are broadcast and the verdicts balloted
+// (256 queries: 8 us; each thread walking all queries' descriptors: 70 us).
+__global__ void batch_mask_kernel(const __grid_constant__ BatchPlan P, int tasks) {
+  const int lane = threadIdx.x & 31;
+  for (int task = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; task < tasks; task += (gridDim.x * blockDim.x) >> 5) {
+    int rest = task, first = 0, last = 0;  // the table's attributes
+    for (;; first = last + 1) {
+      last = first;
+      while (!P.at[last].last) ++last;
+      const int of_table = (P.at[last].ent + 31) / 32 * P.nwords;
+      if (rest < of_table) break;
+      rest -= of_table;
+    }
+    const int w = rest % P.nwords;
+    const int e = rest / P.nwords * 32 + lane;
+    // lane's query: its range on each attribute (all its predicates on one hold together)
+    const int qi = 32 * w + lane;
+    int lo[kMaxComponents], hi[kMaxComponents];
+    unsigned constrains = 0;
+#pragma unroll
+    for (int c = 0; c < kMaxComponents; ++c) {
+      lo[c] = INT_MIN;
+      hi[c] = INT_MAX;
+    }
+    if (qi < P.nq) {
+      const BQ& Q = P.q[qi];
+      for (int p = 0; p < Q.np; ++p) {
+        const int code = Q.pf[p], plo = Q.plo[p], phi = Q.phi[p];
+#pragma unroll
+        for (int c = 0; c < kMaxComponents; ++c)
+          if (first + c <= last && code == P.at[first + c].code) {
+            lo[c] = max(lo[c], plo);
+            hi[c] = min(hi[c], phi);
+            constrains |= 1u << c;
+          }
+      }
+    }
+    // lane's entry: the attributes' values (an interval's verdicts are those of its first value)
+    int x[kMaxComponents];
+    unsigned outside = 0;
+#pragma unroll
+    for (int c = 0; c < kMaxComponents; ++c) {
+      x[c] = 0;
+      if (first + c > last) continue;
+      const Attr& A = P.at[first + c];
+      const int n = A.nint > 0 ? A.nint : A.n;
+      const int i = e / A.mul % (n + 1);
+      if (i == n) outside |= 1u << c;
+      x[c] = A.min + (A.nint > 0 && i < n ? P.bp[A.bp_off + i] : i);
+    }
     unsigned bits = 0;
     for (int j = 0; j < 32; ++j) {
-      const int qi = 32 * w + j;
-      if (qi >= P.nq) break;
-      const BQ& Q = P.q[qi];
-      bool ok = true;
-      for (int p = 0; p < Q.np; ++p)
-        if (Q.pf[p] == code && (x < Q.plo[p] || x > Q.phi[p])) ok = false;
-      if (ok) bits |= 1u << j;
+      const unsigned out = __shfl_sync(kFullMask, outside, j);
+      bool ok = qi < P.nq && (out & constrains) == 0;
+#pragma unroll
+      for (int c = 0; c < kMaxComponents; ++c) {
+        if (first + c > last) break;
+        const int v = __shfl_sync(kFullMask, x[c], j);
+        ok = ok && (!((constrains >> c) & 1u) || (v >= lo[c] && v <= hi[c]));
+      }
+      const unsigned b = __ballot_sync(kFullMask, ok);
+      if (lane == j) bits = b;
     }
-    P.tables[P.f_goff[f] + v * P.nwords + w] = bits;
+    const Attr& A = P.at[last];
+    if (e < A.ent) {
+      const long long at = P.nwords == 8 ? 4ll * ((w >> 2) * A.ent + e) + (w & 3) : static_cast<long long>(e) * P.nwords + w;
+      P.tables[A.goff + at] = bits;
+    }
   }
 }
 
@@ -680,11 +912,12 @@ int batch_init_device(const DeviceState& ds) {
 }
 
 // Fill everything but the shared-memory layout; returns MB_OK or an error.
-static int plan_batch(const mb_batch_args* a, BatchPlan& P) {
+// `sizing`: only what the workspace size needs (the queries keep the caller's order).
+static int plan_batch(const mb_batch_args* a, BatchPlan& P, bool sizing) {
   if (a == nullptr || a->num_queries < 1 || a->num_queries > MB_BATCH_MAX_QUERIES || a->queries == nullptr)
     return MB_ERR_ARG;
   if (a->num_rows < 0) return MB_ERR_ARG;
-  memset(&P, 0, sizeof(P));
+  memset(&P, 0, offsetof(BatchPlan, q));  // the queries' descriptors are cleared one by one below
   P.n = a->num_rows;
   P.nq = a->num_queries;
   // mask words per entry, rounded to 1, 2, 4 or 8 so table entries stay 16-byte aligned
@@ -705,9 +938,11 @@ static int plan_batch(const mb_batch_args* a, BatchPlan& P) {
   };
   // row-schema codes of the aggregation fields, converted to stage codes below
   int af[MB_BATCH_MAX_QUERIES][2], kf[MB_BATCH_MAX_QUERIES][2];
+  unsigned req[MB_BATCH_MAX_QUERIES];  // dims_required
   for (int qi = 0; qi < P.nq; ++qi) {
     const mb_batch_query& q = a->queries[qi];
     BQ& d = P.q[qi];
+    d = BQ{};
     if (q.num_preds < 0 || q.num_preds > MB_BATCH_MAX_PREDS || q.num_keys < 0 || q.num_keys > 2) return MB_ERR_ARG;
     if (q.agg_op < MB_AGG_SUM || q.agg_op > MB_AGG_MUL || q.res == nullptr) return MB_ERR_ARG;
     if (q.res_layout != MB_RES_SCALAR && q.res_layout != MB_RES_CRYSTAL4 && q.res_layout != MB_RES_DENSE)
@@ -741,20 +976,73 @@ static int plan_batch(const mb_batch_args* a, BatchPlan& P) {
                    (nk > 1 ? static_cast<unsigned>(q.key_min[1]) * A.kmul1 : 0u));
     A.total = q.res_layout == MB_RES_SCALAR ? 1 : q.total_val;
     A.soff = -1;
-    A.flags = q.agg_op | ((q.res_layout == MB_RES_CRYSTAL4 ? 1 : 0) << 2) | (nk << 3) | (1 << 8);
+    A.flags = q.agg_op | ((q.res_layout == MB_RES_CRYSTAL4 ? 1 : 0) << 2) | (nk << 3) |
+              ((q.res_layout == MB_RES_SCALAR ? 1 : 0) << 5) | (1 << 8);
     d.res = q.res;
+    req[qi] = static_cast<unsigned>(q.dims_required);
+  }
+  // Classes: queries that add the same expression to the same group index, most members
+  // first. The queries are renumbered class by class, so that a class's bits share few words.
+  int cls_of[MB_BATCH_MAX_QUERIES], first_of[MB_BATCH_MAX_QUERIES], members[MB_BATCH_MAX_QUERIES], nfound = 0;
+  for (int qi = 0; qi < P.nq && !sizing; ++qi) {
+    auto same = [&](int o) {
+      const AQ &A = P.q[qi].a, &C = P.q[o].a;
+      return af[qi][0] == af[o][0] && af[qi][1] == af[o][1] && kf[qi][0] == kf[o][0] && kf[qi][1] == kf[o][1] &&
+             A.kmul0 == C.kmul0 && A.kmul1 == C.kmul1 && A.bias == C.bias && A.total == C.total && A.flags == C.flags;
+    };
+    int c = 0;
+    while (c < nfound && !same(first_of[c])) ++c;
+    if (c == nfound) {
+      first_of[nfound] = qi;
+      members[nfound++] = 0;
+    }
+    ++members[c];
+    cls_of[qi] = c;
+  }
+  if (!sizing) {
+    int rank[MB_BATCH_MAX_QUERIES], order[MB_BATCH_MAX_QUERIES], next[kMaxClasses + 1] = {0};
+    for (int c = 0; c < nfound; ++c) rank[c] = kMaxClasses;
+    for (int i = 0; i < kMaxClasses && i < nfound; ++i) {
+      int best = -1;
+      for (int c = 0; c < nfound; ++c)
+        if (rank[c] == kMaxClasses && (best < 0 || members[c] > members[best])) best = c;
+      rank[best] = i;
+    }
+    for (int qi = 0; qi < P.nq; ++qi) {
+      cls_of[qi] = rank[cls_of[qi]];
+      for (int c = cls_of[qi] + 1; c <= kMaxClasses; ++c) ++next[c];
+    }
+    for (int qi = 0; qi < P.nq; ++qi) order[next[cls_of[qi]]++] = qi;
+    P.ncls = nfound < kMaxClasses ? nfound : kMaxClasses;
+    P.others = nfound > kMaxClasses ? 1 : 0;
+    std::vector<BQ> q0(P.q, P.q + P.nq);
+    std::vector<int> from(6 * P.nq);
+    for (int qi = 0; qi < P.nq; ++qi) {
+      int* f = &from[6 * qi];
+      f[0] = af[qi][0], f[1] = af[qi][1], f[2] = kf[qi][0], f[3] = kf[qi][1];
+      f[4] = static_cast<int>(req[qi]), f[5] = cls_of[qi];
+    }
+    for (int qi = 0; qi < P.nq; ++qi) {
+      const int* f = &from[6 * order[qi]];
+      P.q[qi] = q0[order[qi]];
+      af[qi][0] = f[0], af[qi][1] = f[1], kf[qi][0] = f[2], kf[qi][1] = f[3];
+      req[qi] = static_cast<unsigned>(f[4]), cls_of[qi] = f[5];
+      P.cls_mask[cls_of[qi]][qi / 32] |= 1u << (qi % 32);
+      P.all[qi / 32] |= 1u << (qi % 32);
+    }
   }
   // constrained attributes and the hull of the ranges on each
+  Attr attr[kMaxPredFields] = {};
   int hmin[kMaxPredFields], hmax[kMaxPredFields];
   bool has[kMaxPredFields] = {false};
   for (int qi = 0; qi < P.nq; ++qi) {
     const BQ& d = P.q[qi];
     for (int p = 0; p < d.np; ++p) {
       int f = 0;
-      while (f < P.nfields && P.f_code[f] != d.pf[p]) ++f;
+      while (f < P.nfields && attr[f].code != d.pf[p]) ++f;
       if (f == P.nfields) {
         if (P.nfields == kMaxPredFields) return MB_ERR_SIZE;
-        P.f_code[P.nfields++] = d.pf[p];
+        attr[P.nfields++].code = d.pf[p];
       }
       if (d.plo[p] > d.phi[p]) continue;  // an empty range accepts nothing, inside or outside the hull
       if (!has[f]) {
@@ -767,58 +1055,55 @@ static int plan_batch(const mb_batch_args* a, BatchPlan& P) {
       }
     }
   }
-  long long entries = 0;
   int nbp = 0;
   for (int f = 0; f < P.nfields; ++f) {
+    Attr& A = attr[f];
     const long long n = has[f] ? static_cast<long long>(hmax[f]) - hmin[f] + 1 : 1;
     if (n > 65536) return MB_ERR_SIZE;  // attribute ranges wider than 65,536 values
-    P.f_min[f] = has[f] ? hmin[f] : 0;
-    P.f_n[f] = static_cast<int>(n);
-    P.f_ent[f] = P.f_n[f];
+    A.min = has[f] ? hmin[f] : 0;
+    A.n = static_cast<int>(n);
     if (n > kSmemTableMaxEntries) {
-      // interval coding: end points lo and hi + 1 of every non-empty range on f, and 0
-      int pts[2 * MB_BATCH_MAX_QUERIES * MB_BATCH_MAX_PREDS + 1];
-      int np = 0;
-      pts[np++] = 0;
+      // interval coding: end points lo and hi + 1 of every non-empty range on f, and 0; the
+      // hull has at most 65,536 values, so a bit per value sorts them
+      uint64_t at[65536 / 64] = {0};
+      at[0] = 1;
       for (int qi = 0; qi < P.nq; ++qi) {
         const BQ& d = P.q[qi];
         for (int p = 0; p < d.np; ++p) {
-          if (d.pf[p] != P.f_code[f] || d.plo[p] > d.phi[p]) continue;
-          const long long lo = static_cast<long long>(d.plo[p]) - P.f_min[f];
-          const long long hi1 = static_cast<long long>(d.phi[p]) + 1 - P.f_min[f];
-          if (lo > 0) pts[np++] = static_cast<int>(lo);
-          if (hi1 < n) pts[np++] = static_cast<int>(hi1);
+          if (d.pf[p] != A.code || d.plo[p] > d.phi[p]) continue;
+          const long long lo = static_cast<long long>(d.plo[p]) - A.min;
+          const long long hi1 = static_cast<long long>(d.phi[p]) + 1 - A.min;
+          at[lo / 64] |= 1ull << (lo % 64);
+          if (hi1 < n) at[hi1 / 64] |= 1ull << (hi1 % 64);
         }
       }
-      std::sort(pts, pts + np);
-      np = static_cast<int>(std::unique(pts, pts + np) - pts);
+      int np = 0;
+      for (int i = 0; i < (A.n + 63) / 64; ++i) np += __builtin_popcountll(at[i]);
       if (nbp + np <= kMaxBreakpoints) {
-        P.f_nint[f] = np;
-        P.f_bp_off[f] = nbp;
-        for (int i = 0; i < np; ++i) P.bp[nbp + i] = pts[i];
+        int* bp = P.bp + nbp;
+        for (int i = 0; i < (A.n + 63) / 64; ++i)
+          for (uint64_t w = at[i]; w != 0; w &= w - 1) *bp++ = 64 * i + __builtin_ctzll(w);
+        A.nint = np;
+        A.bp_off = nbp;
         nbp += np;
         int shift = 0;
         while ((static_cast<long long>(kMaxBuckets) << shift) < n) ++shift;
-        P.f_shift[f] = shift;
-        P.f_ent[f] = np;
+        A.bkt_shift = shift;
       }
     }
-    P.f_goff[f] = entries * P.nwords;
-    entries += P.f_ent[f];
   }
-  P.table_entries = entries;
-  // values outside a hull fail every query constraining that attribute
-  for (int f = 0; f < P.nfields; ++f)
+  if (!sizing) {
+    unsigned by_req[16][kMaskWordsMax] = {{0}};
+    unsigned seen = 0;
     for (int qi = 0; qi < P.nq; ++qi) {
-      bool constrains = false;
-      for (int p = 0; p < P.q[qi].np; ++p) constrains = constrains || P.q[qi].pf[p] == P.f_code[f];
-      if (!constrains) P.outside[f][qi / 32] |= 1u << (qi % 32);
+      by_req[req[qi]][qi / 32] |= 1u << (qi % 32);
+      seen |= 1u << req[qi];
     }
-  for (int pm = 0; pm < 16; ++pm)
-    for (int qi = 0; qi < P.nq; ++qi) {
-      const unsigned req = static_cast<unsigned>(a->queries[qi].dims_required);
-      if ((pm & req) == req) P.pres_mask[pm][qi / 32] |= 1u << (qi % 32);
-    }
+    for (unsigned pm = 0; pm < 16; ++pm)
+      for (unsigned r = 0; r < 16; ++r)
+        if (((seen >> r) & 1u) && (pm & r) == r)
+          for (int w = 0; w < P.nwords; ++w) P.pres_mask[pm][w] |= by_req[r][w];
+  }
 
   // dimensions: their keys are staged, their words overwrite the key columns (the date
   // word gets its own column because orderdate is also a field)
@@ -848,13 +1133,17 @@ static int plan_batch(const mb_batch_args* a, BatchPlan& P) {
   }
   for (int d = 0; d < 4; ++d) {
     if (!(dims_used & (1u << d))) continue;
-    P.dim_list[P.ndims++] = d;
-    P.key_stage[d] = P.cidx[kKeyCol[d]];
-    P.pat[d] = a->dim[d].words;
-    P.pat_slots[d] = a->dim[d].slots;
-    P.pat_kmin[d] = a->dim[d].key_min;
-    P.cidx[MB_COL_DIM_S + d] = d == 3 ? P.ncols : P.key_stage[d];
-    P.stage_dim[P.cidx[MB_COL_DIM_S + d]] = d;
+    Dim& D = P.dim[P.ndims++];
+    const int key_stage = P.cidx[kKeyCol[d]];
+    const int word_stage = d == 3 ? P.ncols : key_stage;
+    P.cidx[MB_COL_DIM_S + d] = word_stage;
+    P.stage_dim[word_stage] = d;
+    D.d = d;
+    D.key_word = key_stage;  // columns here; word offsets once the tile is known
+    D.word = word_stage;
+    D.pat = a->dim[d].words;
+    D.slots = a->dim[d].slots;
+    D.kmin = a->dim[d].key_min;
   }
   // a dimension word that replaces its key makes that key unavailable as a field
   auto uses_key = [&](int code) {
@@ -872,7 +1161,7 @@ static int plan_batch(const mb_batch_args* a, BatchPlan& P) {
   }
   // stage codes
   auto scode = [&](int code) { return (P.cidx[code >> 11] << 11) | (code & 0x7ff); };
-  for (int f = 0; f < P.nfields; ++f) P.f_scode[f] = scode(P.f_code[f]);
+  for (int f = 0; f < P.nfields; ++f) attr[f].scode = scode(attr[f].code);
   for (int qi = 0; qi < P.nq; ++qi) {
     AQ& A = P.q[qi].a;
     A.a0 = static_cast<uint16_t>(scode(af[qi][0]));
@@ -880,6 +1169,72 @@ static int plan_batch(const mb_batch_args* a, BatchPlan& P) {
     A.k0 = static_cast<uint16_t>(scode(kf[qi][0]));
     A.k1 = static_cast<uint16_t>(scode(kf[qi][1]));
   }
+  // Position among the batch's dimensions of the one a field reads, -1 for a fact column.
+  int pos_of[MB_NUM_FACT_COLS + 4];
+  for (int& p : pos_of) p = -1;
+  for (int j = 0; j < P.ndims; ++j) pos_of[MB_COL_DIM_S + P.dim[j].d] = j;
+  auto dim_pos = [&](int code) { return pos_of[code >> 11]; };
+  for (int qi = 0; qi < P.nq && !sizing; ++qi) {
+    const unsigned bit = 1u << (qi % 32);
+    const int w = qi / 32;
+    auto uses = [&](int code) {
+      const int j = dim_pos(code);
+      if (j >= 0) P.dim[j].use[w] |= bit;
+    };
+    for (int j = 0; j < P.ndims; ++j)
+      if ((req[qi] >> P.dim[j].d) & 1u) {
+        P.dim[j].need[w] |= bit;
+        P.dim[j].use[w] |= bit;
+      }
+    for (int p = 0; p < P.q[qi].np; ++p) uses(P.q[qi].pf[p]);
+    for (int k = 0; k < 2; ++k) {
+      uses(af[qi][k]);
+      uses(kf[qi][k]);
+    }
+  }
+  // Tables: fact attributes among themselves and dimension attributes among themselves share
+  // one while the product of their index counts stays small (fewer lookups and ANDs per row
+  // for a few KB of shared memory).
+  auto of_dim = [&](int f) { return dim_pos(attr[f].code) >= 0; };
+  auto indexes = [&](int f) { return (attr[f].nint > 0 ? attr[f].nint : attr[f].n) + 1; };
+  int order[kMaxPredFields];
+  for (int f = 0; f < P.nfields; ++f) order[f] = f;
+  std::stable_sort(order, order + P.nfields, [&](int x, int y) {
+    return of_dim(x) != of_dim(y) ? of_dim(x) < of_dim(y) : indexes(x) > indexes(y);
+  });
+  int tab[kMaxPredFields], ntabs = 0, t_ent[kMaxPredFields], t_n[kMaxPredFields];
+  bool t_dim[kMaxPredFields];
+  for (int i = 0; i < P.nfields; ++i) {
+    const int f = order[i];
+    int t = 0;
+    while (t < ntabs && !(t_dim[t] == of_dim(f) && t_n[t] < kMaxComponents &&
+                          static_cast<long long>(t_ent[t]) * indexes(f) <= kCombineMaxEntries))
+      ++t;
+    if (t == ntabs) {
+      t_dim[t] = of_dim(f);
+      t_ent[t] = 1;
+      t_n[t] = 0;
+      ++ntabs;
+    }
+    attr[f].mul = t_ent[t];
+    t_ent[t] *= indexes(f);
+    ++t_n[t];
+    tab[f] = t;
+  }
+  std::stable_sort(order, order + P.nfields, [&](int x, int y) { return tab[x] < tab[y]; });
+  long long entries = 0;
+  for (int i = 0; i < P.nfields; ++i) {
+    const int f = order[i];
+    Attr& A = P.at[i];
+    A = attr[f];
+    if (!of_dim(f)) P.nfact = i + 1;
+    A.last = i + 1 == P.nfields || tab[order[i + 1]] != tab[f] ? 1 : 0;
+    if (!A.last) continue;
+    A.ent = t_ent[tab[f]];
+    A.goff = entries * P.nwords;
+    entries += A.ent;
+  }
+  P.table_entries = entries;
   return MB_OK;
 }
 
@@ -912,7 +1267,7 @@ extern "C" size_t mb_batch_workspace_bytes(const mb_batch_args* a) {
   static BatchPlan P;  // large; host-side scratch for sizing only
   static std::mutex mu;
   std::lock_guard<std::mutex> lk(mu);
-  if (plan_batch(a, P) != MB_OK) return 0;
+  if (plan_batch(a, P, true) != MB_OK) return 0;
   return workspace_bytes(P);
 }
 
@@ -923,7 +1278,7 @@ extern "C" int mb_batch_run(const mb_batch_args* a, mb_stream_t stream) {
     ~Free() { delete p; }
   } guard{Pp};
   BatchPlan& P = *Pp;
-  int e = plan_batch(a, P);
+  int e = plan_batch(a, P, false);
   if (e != MB_OK) return e;
   if (P.n == 0) return MB_OK;
   if (workspace_bytes(P) > 0 &&
@@ -935,9 +1290,14 @@ extern "C" int mb_batch_run(const mb_batch_args* a, mb_stream_t stream) {
   if (ds == nullptr) return err;
   P.status = ds->status;
 
-  // defaults measured best for 256 queries over 120M rows: 24 consumer warps, one row a lane
-  const int threads = a->threads ? a->threads : 768;
-  const int items = a->items_per_thread ? a->items_per_thread : 1;
+  // Defaults: up to 64 queries a row has few matches and the work per row decides, so a lane
+  // takes two rows at a time (24 queries over 75 M rows: 768x2 1.76 ms, 960x1 2.22, 768x1
+  // 2.52); above, the match lists are full anyway and one more warp a scheduler hides more
+  // (120 queries over 20 M rows: 960x1 1.10 ms, 768x1 1.20, 768x2 1.33; 256 queries: 2.21,
+  // 2.30, 2.21). A call that sets one of the two gets 768 threads or one row for the other.
+  const bool by_size = a->threads == 0 && a->items_per_thread == 0;
+  const int threads = a->threads ? a->threads : by_size && P.nwords > 2 ? 960 : 768;
+  const int items = a->items_per_thread ? a->items_per_thread : by_size && P.nwords <= 2 ? 2 : 1;
   const int nwm = P.nwords;
   const BatchVariant* var = nullptr;
   for (const BatchVariant& v : kBatchVariants)
@@ -945,13 +1305,30 @@ extern "C" int mb_batch_run(const mb_batch_args* a, mb_stream_t stream) {
   if (var == nullptr) return MB_ERR_ARG;
   const int tile = threads * items;
   P.nfull = P.n / tile;
-  P.stage_words = (P.ncols + ((P.ndims && P.dim_list[P.ndims - 1] == 3) ? 1 : 0)) * (tile + kColPad);
+  // stage word offsets
+  auto field = [&](int code) {
+    const int width = code & 63;
+    return Field{(code >> 11) * (tile + kColPad), (code >> 6) & 31, width >= 32 ? 0xffffffffu : (1u << width) - 1u};
+  };
+  for (int f = 0; f < P.nfields; ++f) P.at[f].f = field(P.at[f].scode);
+  for (int j = 0; j < P.ndims; ++j) {
+    P.dim[j].key_word *= tile + kColPad;
+    P.dim[j].word *= tile + kColPad;
+  }
+  for (int c = 0; c < P.ncls; ++c) {
+    int qi = 0;  // its first query
+    while (!((P.cls_mask[c][qi / 32] >> (qi % 32)) & 1u)) ++qi;
+    const AQ& A = P.q[qi].a;
+    P.cls[c] = {field(A.a0), field(A.a1), field(A.k0), field(A.k1), A.kmul0, A.kmul1, A.bias,
+                A.total, A.flags & 3, (A.flags >> 5) & 1, ((A.flags >> 3) & 3) > 1 ? 1 : 0};
+  }
+  P.stage_words = (P.ncols + ((P.ndims && P.dim[P.ndims - 1].d == 3) ? 1 : 0)) * (tile + kColPad);
   int stages = a->stages ? a->stages : 2;
   if (stages < 2 || stages > kBatchStages) return MB_ERR_ARG;
 
-  // shared memory: barriers | scalars | aggregation descriptors | result pointers |
-  // presence masks | outside masks | small predicate tables | match lists |
-  // small group arrays | stage ring
+  // shared memory: barriers | scalars | aggregation descriptors | match records | result
+  // pointers | sum addresses | presence masks | predicate tables | match lists | small
+  // group arrays | stage ring
   int off = 2 * kBatchStages * 8;
   int nscalar = 0;
   for (int qi = 0; qi < P.nq; ++qi) nscalar += P.q[qi].res_layout == MB_RES_SCALAR ? 1 : 0;
@@ -961,35 +1338,34 @@ extern "C" int mb_batch_run(const mb_batch_args* a, mb_stream_t stream) {
   off = (off + 15) / 16 * 16;
   P.smem_aq_off = off;
   off += static_cast<int>(sizeof(AQ)) * P.nq;
+  P.smem_qd_off = off;
+  off += static_cast<int>(sizeof(QD)) * P.nq;
   P.smem_res_off = off;
+  off += 8 * P.nq;
+  P.smem_addr_off = off;
   off += 8 * P.nq;
   off = (off + 15) / 16 * 16;
   P.smem_pres_off = off;
   off += 16 * kMaskWordsMax * 4;
-  P.smem_out_off = off;
-  off += kMaxPredFields * kMaskWordsMax * 4;
-  for (int f = 0; f < P.nfields; ++f) {
-    P.f_smem_off[f] = -1;
-    if (P.f_ent[f] <= kSmemTableMaxEntries || P.f_nint[f] > 0) {
-      P.f_smem_off[f] = off;
-      off += (P.f_ent[f] * P.nwords * 4 + 15) / 16 * 16;
-    }
-    if (P.f_nint[f] > 0) {
-      P.f_bps_off[f] = off;
-      off += (P.f_nint[f] * 4 + 15) / 16 * 16;
-      P.f_bkt_off[f] = off;
-      off += ((((P.f_n[f] - 1) >> P.f_shift[f]) + 1) * 2 + 15) / 16 * 16;
-    }
-  }
-  P.smem_list_off = off;
   const int budget = ds->max_smem_optin - 2048;
   auto total_smem = [&](int base, int st) { return (base + 127) / 128 * 128 + st * P.stage_words * 4; };
-  // match lists: 1,024 pairs a warp, or 512 where that leaves shared-memory group arrays
-  // less than 64 KB (a list must hold the pairs of 32 rows with ease: ~8 queries a row
-  // pass on average in a batch of 256 with log-uniform selectivities up to 0.3)
-  P.list_cap = kMatchListMax;
-  if (total_smem(off + (threads / 32) * P.list_cap * 4, stages) > budget - 65536) P.list_cap = 512;
-  off += (threads / 32) * P.list_cap * 4;
+  for (int f = 0; f < P.nfields; ++f) {
+    Attr& A = P.at[f];
+    if (A.nint > 0) {
+      A.bps_off = off;
+      off += (A.nint * 4 + 15) / 16 * 16;
+      A.bkt_off = off;
+      off += ((((A.n - 1) >> A.bkt_shift) + 1) * 2 + 15) / 16 * 16;
+    }
+    if (!A.last) continue;
+    // single attributes with too many values and end points stay in the workspace
+    A.smem_off = -1;
+    if (A.nint == 0 && A.ent > kSmemTableMaxEntries + 1) continue;
+    A.smem_off = off;
+    off += (A.ent * P.nwords * 4 + 15) / 16 * 16;
+  }
+  P.smem_list_off = off;
+  off += (threads / 32) * kMatchListCap * 2;
   while (total_smem(off, stages) > budget && stages > 2) --stages;
   if (total_smem(off, stages) > budget) return MB_ERR_SIZE;
   P.stages = stages;
@@ -997,7 +1373,6 @@ extern "C" int mb_batch_run(const mb_batch_args* a, mb_stream_t stream) {
   for (int qi = 0, k = 0; qi < P.nq; ++qi)
     if (P.q[qi].res_layout == MB_RES_SCALAR) {
       P.q[qi].a.soff = P.smem_acc_off + 8 * kScalarCopies * k++;
-      P.q[qi].a.flags |= 1 << 5;
     }
   // small group arrays (<= 1,024 groups) to shared memory, smallest first, within the budget
   P.smem_groups_off = off;
@@ -1068,17 +1443,20 @@ extern "C" int mb_batch_run(const mb_batch_args* a, mb_stream_t stream) {
 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (P.table_entries > 0) {
-    const long long work = P.table_entries * P.nwords;
-    long long blocks = (work + 255) / 256;
+    long long tasks = 0;  // warps' worth: 32 entries of a table, one word
+    for (int f = 0; f < P.nfields; ++f) tasks += P.at[f].last ? (P.at[f].ent + 31) / 32 * P.nwords : 0;
+    long long blocks = (tasks + 3) / 4;
     if (blocks > ds->num_sms * 8) blocks = ds->num_sms * 8;
-    batch_mask_kernel<<<static_cast<int>(blocks), 256, 0, st>>>(P);
+    batch_mask_kernel<<<static_cast<int>(blocks), 128, 0, st>>>(P, static_cast<int>(tasks));
     if (cudaGetLastError() != cudaSuccess) return MB_ERR_LAUNCH;
     note_launches(1);
   }
   int grid = a->grid;
   if (grid <= 0) {
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, var->fn, threads + 32, smem) != cudaSuccess)
+    // 16 warps or more leave registers for one CTA an SM; only the 8-warp shapes have to ask
+    int per_sm = 1;
+    if (threads < 512 &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, var->fn, threads + 32, smem) != cudaSuccess)
       return MB_ERR_CUDA;
     grid = ds->num_sms * (per_sm < 1 ? 1 : per_sm);
   }
