@@ -16,18 +16,31 @@
 // takes the group value an earlier join found: the dimension column `ht` read at the
 // dimension row fkey[k] (BlockReadFilteredOffset, BlockLibrary.cuh:484-541).
 //
-// The rows of a list are gathers, not a stream, so this kernel is a plain grid-stride loop
-// (each thread keeps kListItems rows in flight) with the star kernel's group accumulation:
-// 64-bit sums in a shared-memory group array flushed once per CTA, or L2 atomics for large
-// group arrays; scalars reduced per CTA.
+// The rows of a list are gathers, not a stream, so the kernel is bound by how many loads it
+// has in flight and how long its chain of dependent ones is. A thread keeps kListItems
+// entries and runs them through straight-line rounds (every load of a round goes out before
+// one is used): the entries' rows; the filters; the first table probe; then the remaining
+// probes of its survivors — and, when that is one table at most, the aggregate columns with
+// them; at last the passed-through group values and the aggregates. Outcomes are combined
+// probe by probe in the chain's order, so selection and status bits equal the sequential
+// chain's. Group accumulation is the star kernel's: 64-bit sums in a shared-memory group
+// array flushed once per CTA, or L2 atomics for large group arrays; scalars reduced per CTA.
+// 2,000,003 entries over 24,000,000 rows (segment cache, two table probes, one passed-through
+// value): one entry at a time behind branches 127 us; in rounds 76 us. Its entries lie 12 rows
+// apart, so the four gathered columns come in nearly whole (343 MB, 52 us at the copy rate).
 #include <cstring>
+#include <type_traits>
 
 #include "star.cuh"
 
 namespace mb {
 
-constexpr int kListItems = 4;
+// Two entries a thread at three CTAs an SM is what the registers carry without spilling
+// (2,000,003 entries: 81 us a call; 4 entries at 3 CTAs 113 us and 2 at 4 CTAs 93 us, both
+// spilling; 4 at 2 CTAs 80 us, but 133 against 123 us for 4.8 M entries).
+constexpr int kListItems = 2;
 constexpr int kListThreads = 256;
+constexpr int kListCtas = 3;
 
 struct ListPlan {
   long long n;
@@ -60,38 +73,6 @@ __device__ __forceinline__ bool list_pass(int x, int mode, int c1, int c2) {
   return x == c1 || x == c2;
 }
 
-// Where row k of the call lives: (segment, in-segment row) under segment addressing,
-// (-1, column index) otherwise.
-__device__ __forceinline__ void list_locate(const ListPlan& P, long long k, int& seg, long long& idx) {
-  const long long phys = P.rows ? static_cast<long long>(__ldg(P.rows + k)) : k;
-  if (P.gpu_cache == nullptr) {
-    seg = -1;
-    idx = phys;
-    return;
-  }
-  const long long mask = (1ll << P.seg_shift) - 1;
-  if (P.rows) {
-    seg = static_cast<int>(phys >> P.seg_shift);  // physical rows index the slot arrays directly
-  } else {
-    const long long vseg = k >> P.seg_shift;
-    seg = P.seg_group ? static_cast<int>(P.seg_group[vseg]) : static_cast<int>((P.start_offset + k) >> P.seg_shift);
-  }
-  idx = phys & mask;
-}
-
-__device__ __forceinline__ int list_read(const ListPlan& P, const int* col, int seg, long long idx) {
-  if (P.gpu_cache == nullptr) return __ldg(col + idx);
-  return __ldg(P.gpu_cache + (static_cast<long long>(__ldg(col + seg)) << P.seg_shift) + idx);
-}
-
-// A dimension column at dimension row d (direct, or through the segment cache).
-__device__ __forceinline__ int list_read_dim(const ListPlan& P, const int* col, int d) {
-  if (P.gpu_cache == nullptr) return __ldg(col + d);
-  const int seg = d >> P.seg_shift;
-  return __ldg(P.gpu_cache + (static_cast<long long>(__ldg(col + seg)) << P.seg_shift) +
-               (d & ((1 << P.seg_shift) - 1)));
-}
-
 __device__ __forceinline__ unsigned long long* list_sum_ptr(const ListPlan& P, int h) {
   if (P.res_layout == MB_RES_ENGINE6)
     return reinterpret_cast<unsigned long long*>(static_cast<int*>(P.res) + 6 * h + 4);
@@ -100,14 +81,11 @@ __device__ __forceinline__ unsigned long long* list_sum_ptr(const ListPlan& P, i
   return static_cast<unsigned long long*>(P.res) + h;
 }
 
-__device__ __forceinline__ void list_keys(const ListPlan& P, int h, const int (&gv)[MB_MAX_PROBES]) {
-  int* res = static_cast<int*>(P.res);
-  const int stride = P.res_layout == MB_RES_ENGINE6 ? 6 : 4;
-  for (int p = 0; p < P.np; ++p)
-    if (P.p_res_slot[p] >= 0) res[stride * h + P.p_res_slot[p]] = gv[p];
-}
-
-__global__ void __launch_bounds__(kListThreads) list_kernel(const __grid_constant__ ListPlan P) {
+// SEG: segment-cache addressing (gpu_cache set).
+template <bool SEG>
+__global__ void __launch_bounds__(kListThreads, kListCtas) list_kernel(const __grid_constant__ ListPlan P) {
+  constexpr int R = kListItems;
+  using Index = std::conditional_t<SEG, int, long long>;  // in-segment row, or row of the column
   extern __shared__ __align__(16) unsigned char lsmem[];
   __shared__ unsigned long long s_red[2 * kListThreads / 32];
   unsigned long long* s_sum = reinterpret_cast<unsigned long long*>(lsmem);
@@ -120,101 +98,207 @@ __global__ void __launch_bounds__(kListThreads) list_kernel(const __grid_constan
   __syncthreads();
   unsigned long long acc = 0, cnt = 0;
   bool bad_probe = false, bad_group = false;
+  // the first table probe; a second round follows it, with the aggregate columns when it
+  // holds one table at most
+  int first = 0, later_tables = 0;
+  while (first < P.np && P.p_layout[first] == MB_HT_PASS) ++first;
+  for (int p = first + 1; p < P.np; ++p) later_tables += P.p_layout[p] != MB_HT_PASS ? 1 : 0;
+  const bool early_aggr = later_tables <= 1;
+  const bool two_cols = P.agg_op == MB_AGG_SUB || P.agg_op == MB_AGG_MUL;
   const long long stride = static_cast<long long>(gridDim.x) * kListThreads;
-  for (long long base = blockIdx.x * static_cast<long long>(kListThreads) * kListItems + tid; base < P.n;
-       base += stride * kListItems) {
-    // kListItems rows a thread, k = base + i * kListThreads: their gathers are independent
-    int seg[kListItems];
-    long long idx[kListItems];
-    bool ok[kListItems];
+  for (long long base = blockIdx.x * static_cast<long long>(kListThreads) * R + tid; base < P.n; base += stride * R) {
+    // ---- entries k = base + i * kListThreads: their rows ----
+    int seg[R];
+    Index idx[R];
+    unsigned sel = 0;
 #pragma unroll
-    for (int i = 0; i < kListItems; ++i) {
+    for (int i = 0; i < R; ++i) {
       const long long k = base + static_cast<long long>(i) * kListThreads;
-      ok[i] = k < P.n;
-      seg[i] = 0;
-      idx[i] = 0;
-      if (ok[i]) list_locate(P, k, seg[i], idx[i]);
-    }
-    for (int f = 0; f < P.nf; ++f) {
-#pragma unroll
-      for (int i = 0; i < kListItems; ++i) {
-        if (P.count_after == f && ok[i]) ++cnt;
-        if (ok[i]) ok[i] = list_pass(list_read(P, P.f_col[f], seg[i], idx[i]), P.f_mode[f], P.f_c1[f], P.f_c2[f]);
+      seg[i] = idx[i] = 0;
+      if (k < P.n) {
+        sel |= 1u << i;
+        if (P.rows) {
+          idx[i] = __ldg(P.rows + k);
+        } else {
+          idx[i] = static_cast<Index>(SEG ? k & ((1ll << P.seg_shift) - 1) : k);
+          if (SEG)
+            seg[i] = P.seg_group ? static_cast<int>(P.seg_group[k >> P.seg_shift])
+                                 : static_cast<int>((P.start_offset + k) >> P.seg_shift);
+        }
       }
     }
-    if (P.count_after >= P.nf) {
+    if (SEG && P.rows) {
 #pragma unroll
-      for (int i = 0; i < kListItems; ++i) cnt += ok[i];
+      for (int i = 0; i < R; ++i) {
+        seg[i] = static_cast<int>(idx[i] >> P.seg_shift);  // physical rows index the slot arrays directly
+        idx[i] &= (1 << P.seg_shift) - 1;
+      }
     }
-    int gv[kListItems][MB_MAX_PROBES];
-    for (int p = 0; p < P.np; ++p) {
+    // a column at the entries in `of` (0 elsewhere)
+    auto load = [&](const int* col, unsigned of, int (&v)[R]) {
+      if (SEG) {
 #pragma unroll
-      for (int i = 0; i < kListItems; ++i) {
-        gv[i][p] = 0;
-        if (!ok[i]) continue;
+        for (int i = 0; i < R; ++i) v[i] = (of >> i) & 1u ? __ldg(col + seg[i]) : 0;
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+          v[i] = (of >> i) & 1u ? __ldg(P.gpu_cache + (static_cast<long long>(v[i]) << P.seg_shift) + idx[i]) : 0;
+      } else {
+#pragma unroll
+        for (int i = 0; i < R; ++i) v[i] = (of >> i) & 1u ? __ldg(col + idx[i]) : 0;
+      }
+    };
+    // ---- filters ----
+#pragma unroll
+    for (int f = 0; f < MB_MAX_FILTERS; ++f) {
+      if (f >= P.nf) break;
+      if (P.count_after == f) cnt += __popc(sel);
+      int v[R];
+      load(P.f_col[f], sel, v);
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+        if (!list_pass(v[i], P.f_mode[f], P.f_c1[f], P.f_c2[f])) sel &= ~(1u << i);
+    }
+    if (P.count_after >= P.nf) cnt += __popc(sel);
+    // ---- probes: gv[p] = the payload, or the dimension row of a passed-through value ----
+    int gv[MB_MAX_PROBES][R], a0[R], a1[R];
+#pragma unroll
+    for (int p = 0; p < MB_MAX_PROBES; ++p)
+#pragma unroll
+      for (int i = 0; i < R; ++i) gv[p][i] = 0;
+#pragma unroll
+    for (int i = 0; i < R; ++i) a0[i] = a1[i] = 0;
+    auto round = [&](auto in_round) {
+      unsigned long long sv[MB_MAX_PROBES][R];
+      unsigned range_bad[MB_MAX_PROBES];
+#pragma unroll
+      for (int p = 0; p < MB_MAX_PROBES; ++p) {
+        range_bad[p] = 0;
+        if (p >= P.np || !in_round(p)) continue;
         if (P.p_layout[p] == MB_HT_PASS) {
-          const long long k = base + static_cast<long long>(i) * kListThreads;
-          const int d = __ldg(P.p_key[p] + k);
-          if (d < 0 || d >= P.p_slots[p]) {
-            bad_probe = true;
-            ok[i] = false;
-          } else {
-            gv[i][p] = list_read_dim(P, P.p_ht[p], d);
-          }
+#pragma unroll
+          for (int i = 0; i < R; ++i)
+            if ((sel >> i) & 1u) gv[p][i] = __ldg(P.p_key[p] + base + static_cast<long long>(i) * kListThreads);
+        } else {
+          load(P.p_key[p], sel, gv[p]);
+        }
+      }
+#pragma unroll
+      for (int p = 0; p < MB_MAX_PROBES; ++p) {
+        if (p >= P.np || !in_round(p)) continue;
+        const int layout = P.p_layout[p], slots = P.p_slots[p];
+        if (layout == MB_HT_PASS) {
+#pragma unroll
+          for (int i = 0; i < R; ++i)
+            if (gv[p][i] < 0 || gv[p][i] >= slots) range_bad[p] |= 1u << i;
           continue;
         }
-        const int key = list_read(P, P.p_key[p], seg[i], idx[i]);
-        const int dd = static_cast<int>(static_cast<unsigned>(key) - static_cast<unsigned>(P.p_kmin[p]));
-        const int h = (static_cast<unsigned>(dd) < static_cast<unsigned>(P.p_slots[p])) ? dd : dd % P.p_slots[p];
-        if (h < 0) {
-          bad_probe = true;
-          ok[i] = false;
-        } else if (P.p_layout[p] == MB_HT_KEY) {
-          ok[i] = __ldg(P.p_ht[p] + h) != 0;
+        const int* ht = P.p_ht[p];
+        int h[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+          h[i] = pht_slot(gv[p][i], slots, P.p_kmin[p]);
+          if (h[i] < 0) {
+            range_bad[p] |= 1u << i;
+            h[i] = 0;
+          }
+        }
+        const unsigned of = sel & ~range_bad[p];
+        if (layout == MB_HT_KEY) {
+#pragma unroll
+          for (int i = 0; i < R; ++i) sv[p][i] = (of >> i) & 1u ? static_cast<unsigned>(__ldg(ht + h[i])) : 0u;
         } else {
-          const unsigned long long s = ldg_u64(P.p_ht[p] + 2ll * h);
-          ok[i] = s != 0;
-          gv[i][p] = P.p_layout[p] == MB_HT_KEY_VAL ? static_cast<int>(s >> 32) : static_cast<int>(static_cast<unsigned>(s));
+#pragma unroll
+          for (int i = 0; i < R; ++i) sv[p][i] = (of >> i) & 1u ? ldg_u64(ht + 2ll * h[i]) : 0ull;
         }
       }
-    }
 #pragma unroll
-    for (int i = 0; i < kListItems; ++i) {
-      if (!ok[i]) continue;
-      if (P.count_after < 0) ++cnt;
-      const int a0 = list_read(P, P.a_col[0], seg[i], idx[i]);
-      int val;
-      if (P.agg_op == MB_AGG_SUM) {
-        val = a0;
-      } else if (P.agg_op == MB_AGG_MUL_PAYLOAD) {
-        val = static_cast<int>(static_cast<unsigned>(a0) * static_cast<unsigned>(gv[i][0]));
-      } else {
-        const int a1 = list_read(P, P.a_col[1], seg[i], idx[i]);
-        val = P.agg_op == MB_AGG_SUB ? static_cast<int>(static_cast<unsigned>(a0) - static_cast<unsigned>(a1))
-                                     : static_cast<int>(static_cast<unsigned>(a0) * static_cast<unsigned>(a1));
+      for (int p = 0; p < MB_MAX_PROBES; ++p) {
+        if (p >= P.np || !in_round(p)) continue;
+        if (sel & range_bad[p]) bad_probe = true;
+        sel &= ~range_bad[p];
+        const int layout = P.p_layout[p];
+        if (layout == MB_HT_PASS) continue;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+          if (sv[p][i] == 0) sel &= ~(1u << i);
+          gv[p][i] = layout == MB_HT_KEY_VAL   ? static_cast<int>(sv[p][i] >> 32)
+                     : layout == MB_HT_VAL_OFF ? static_cast<int>(static_cast<unsigned>(sv[p][i]))
+                                               : 0;
+        }
       }
+    };
+    if (P.np > 0) {
+      round([&](int p) { return p <= first; });
+      if (early_aggr) {
+        load(P.a_col[0], sel, a0);
+        if (two_cols) load(P.a_col[1], sel, a1);
+      }
+      round([&](int p) { return p > first; });
+    }
+    if (P.count_after < 0) cnt += __popc(sel);
+    if (!early_aggr || P.np == 0) {
+      load(P.a_col[0], sel, a0);
+      if (two_cols) load(P.a_col[1], sel, a1);
+    }
+    // ---- passed-through group values: the dimension column at the listed dimension row ----
+#pragma unroll
+    for (int p = 0; p < MB_MAX_PROBES; ++p) {
+      if (p >= P.np) break;
+      if (P.p_layout[p] != MB_HT_PASS) continue;
+      const int* col = P.p_ht[p];
+      if (SEG) {
+        int slot[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) slot[i] = (sel >> i) & 1u ? __ldg(col + (gv[p][i] >> P.seg_shift)) : 0;
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+          if ((sel >> i) & 1u)
+            gv[p][i] = __ldg(P.gpu_cache + (static_cast<long long>(slot[i]) << P.seg_shift) +
+                             (gv[p][i] & ((1 << P.seg_shift) - 1)));
+      } else {
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+          if ((sel >> i) & 1u) gv[p][i] = __ldg(col + gv[p][i]);
+      }
+    }
+    // ---- aggregate ----
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      if (!((sel >> i) & 1u)) continue;
+      const unsigned u0 = static_cast<unsigned>(a0[i]), u1 = static_cast<unsigned>(a1[i]);
+      const int val = static_cast<int>(P.agg_op == MB_AGG_SUM           ? u0
+                                       : P.agg_op == MB_AGG_MUL_PAYLOAD ? u0 * static_cast<unsigned>(gv[0][i])
+                                       : P.agg_op == MB_AGG_SUB         ? u0 - u1
+                                                                        : u0 * u1);
       const unsigned long long w = static_cast<unsigned long long>(static_cast<long long>(val));
       if (P.gmode == kGroupScalar) {
         acc += w;
         continue;
       }
       unsigned hh = static_cast<unsigned>(P.group_bias);
-      for (int p = 0; p < P.np; ++p)
-        hh += (static_cast<unsigned>(gv[i][p]) - static_cast<unsigned>(P.p_min[p])) * static_cast<unsigned>(P.p_mul[p]);
-      const int h = static_cast<int>(hh) % P.total_val;
+#pragma unroll
+      for (int p = 0; p < MB_MAX_PROBES; ++p)
+        if (p < P.np)
+          hh += (static_cast<unsigned>(gv[p][i]) - static_cast<unsigned>(P.p_min[p])) * static_cast<unsigned>(P.p_mul[p]);
+      int h = static_cast<int>(hh);
+      if (hh >= static_cast<unsigned>(P.total_val)) h = slow_mod(h, P.total_val);
       if (h < 0) {
         bad_group = true;
         continue;
       }
+      bool keys = P.res_layout != MB_RES_DENSE;
       if (P.gmode == kGroupSmem) {
         smem_add_i64(&s_sum[h], val);
         const uint32_t bit = 1u << (h & 31);
-        if (!(s_touch[h >> 5] & bit) && !(atomicOr(&s_touch[h >> 5], bit) & bit) && P.res_layout != MB_RES_DENSE)
-          list_keys(P, h, gv[i]);
+        keys = !(s_touch[h >> 5] & bit) && !(atomicOr(&s_touch[h >> 5], bit) & bit) && keys;
       } else {
-        if (P.res_layout != MB_RES_DENSE) list_keys(P, h, gv[i]);
         atomicAdd(list_sum_ptr(P, h), w);
       }
+      if (!keys) continue;
+      int* res = static_cast<int*>(P.res) + static_cast<long long>(P.res_layout == MB_RES_ENGINE6 ? 6 : 4) * h;
+#pragma unroll
+      for (int p = 0; p < MB_MAX_PROBES; ++p)
+        if (p < P.np && P.p_res_slot[p] >= 0) res[P.p_res_slot[p]] = gv[p][i];
     }
   }
   if (bad_probe) set_status(P.status, MB_STATUS_PROBE_RANGE);
@@ -245,8 +329,11 @@ __global__ void __launch_bounds__(kListThreads) list_kernel(const __grid_constan
 }
 
 int list_init_device(const DeviceState& ds) {
-  return cuda_status(cudaFuncSetAttribute(reinterpret_cast<const void*>(list_kernel),
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, ds.max_smem_optin - 2048));
+  for (auto fn : {list_kernel<false>, list_kernel<true>})
+    if (cudaFuncSetAttribute(reinterpret_cast<const void*>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             ds.max_smem_optin - 2048) != cudaSuccess)
+      return MB_ERR_CUDA;
+  return MB_OK;
 }
 
 int launch_list(const mb_star_args* a, cudaStream_t stream, const DeviceState* ds) {
@@ -312,10 +399,11 @@ int launch_list(const mb_star_args* a, cudaStream_t stream, const DeviceState* d
   }
   const long long per_block = static_cast<long long>(kListThreads) * kListItems;
   long long blocks = (P.n + per_block - 1) / per_block;
-  const long long cap = static_cast<long long>(ds->num_sms) * 8;
+  const long long cap = static_cast<long long>(ds->num_sms) * kListCtas;
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
-  list_kernel<<<static_cast<int>(blocks), kListThreads, smem, stream>>>(P);
+  const auto fn = P.gpu_cache != nullptr ? list_kernel<true> : list_kernel<false>;
+  fn<<<static_cast<int>(blocks), kListThreads, smem, stream>>>(P);
   if (cudaGetLastError() != cudaSuccess) return MB_ERR_LAUNCH;
   note_launches(1);
   return MB_OK;
