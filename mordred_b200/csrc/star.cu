@@ -52,7 +52,7 @@ int star_init_device(const DeviceState& ds) {
       if (e != cudaSuccess) return MB_ERR_CUDA;
     }
   }
-  return MB_OK;
+  return ring_init_device(ds);
 }
 
 static int add_col(StarPlan& P, const int* c) {
@@ -261,6 +261,19 @@ int launch_star(const mb_star_args* a, cudaStream_t stream, int count32, const D
     P.seg_shift = __builtin_ctz(static_cast<unsigned>(ss));
   }
 
+  // ---- calls with probes and no launch shape of their own -------------------------
+  if (a->mirrors < 0 || a->mirrors > 2) return MB_ERR_ARG;
+  if (a->pack < 0 || a->pack > 4) return MB_ERR_ARG;
+  bool tiles = true;
+  for (int c = 0; c < P.ncols; ++c) tiles = tiles && (P.gpu_cache != nullptr || aligned16(P.col[c]));
+  if (P.np > 0 && a->agg_op != MB_AGG_MUL_PAYLOAD && tiles && P.n < (1ll << 32) &&
+      (P.gpu_cache == nullptr || P.seg_shift >= 8) && a->threads == 0 && a->items_per_thread == 0 && a->stages == 0 &&
+      a->grid == 0 && a->mirrors != 2 && a->pack == 0 && a->group_mode != 1) {
+    const int big = P.res_layout != MB_RES_SCALAR && P.total_val > 2048 ? 2 : 0;
+    const int e = launch_ring(P, a->group_mode ? a->group_mode : big, *ds, stream);
+    if (e != MB_ERR_SIZE) return e;
+  }
+
   // ---- launch configuration and shared-memory plan ------------------------------
   // Unset fields take the tuned configuration for this query shape (tuned_configs.h).
   const TunedConfig tc = tuned_config(P.nf, a->num_probes, a->probe[0].layout, P.res_layout, P.total_val, P.n);
@@ -286,8 +299,6 @@ int launch_star(const mb_star_args* a, cudaStream_t stream, int count32, const D
     P.gmode = P.total_val <= kSmemGroupMax ? kGroupSmem : kGroupGlobal;
   if (group_mode == 1 && P.gmode != kGroupSmem) return MB_ERR_SIZE;
 
-  if (a->mirrors < 0 || a->mirrors > 2) return MB_ERR_ARG;
-  if (a->pack < 0 || a->pack > 4) return MB_ERR_ARG;
   const bool want_pack = a->pack == 2 || a->pack == 3 || (a->pack == 0 && (tc.pack == 1 || tc.pack == 2));
   const bool want_rel = a->pack >= 3 || (a->pack == 0 && tc.pack >= 2);
   const int budget = ds->max_smem_optin - 2048 - 2 * 8 * (ncw + 1);

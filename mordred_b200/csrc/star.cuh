@@ -103,6 +103,10 @@ struct StarPlan {
   int mir_payload[MB_MAX_PROBES];  // 1: the probe's payload is read (from its code, else from the table)
   int mir_shift;
   int smem_mirror_off;
+  // star_ring.cu: staged columns (indexes into col), and which of them each filter, bitmap
+  // probe and the probe before the ring reads
+  int r_nst, r_col[MB_MAX_FILTERS + MB_MAX_PROBES];
+  int r_fcol[MB_MAX_FILTERS], r_pcol[MB_MAX_PROBES], r_kcol;
 };
 
 // Host: validate `a`, fill `plan`, pick the kernel variant and launch it on `stream`.
@@ -112,6 +116,11 @@ int launch_star(const mb_star_args* a, cudaStream_t stream, int count32, const D
 
 // Host: set per-device kernel attributes (dynamic shared memory opt-in).
 int star_init_device(const DeviceState& ds);
+// Host: the default form of calls with probes (star_ring.cu). `plan` holds the validated call
+// (columns 16-byte aligned, fewer than 2^32 rows); group_mode 2 keeps the groups in L2.
+// MB_ERR_SIZE when its shared memory does not fit (nothing was launched).
+int launch_ring(StarPlan& plan, int group_mode, const DeviceState& ds, cudaStream_t stream);
+int ring_init_device(const DeviceState& ds);
 // Host: the offset-list form of the pipeline (listq.cu): a->rows lists physical rows, or a
 // probe passes a group value through (MB_HT_PASS). Arguments are validated here.
 int launch_list(const mb_star_args* a, cudaStream_t stream, const DeviceState* ds);
