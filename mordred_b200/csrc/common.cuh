@@ -17,12 +17,15 @@ static __device__ __noinline__ int slow_mod(int d, int m) { return d % m; }
 
 // ((key - key_min) % slots) in 32-bit two's complement (crystal/join.cuh:3). Keys in
 // [key_min, key_min + slots) map to themselves and the next range wraps by one
-// subtraction (a dense 1-based key N lands on slot 0); only other keys divide.
+// subtraction (a dense 1-based key N lands on slot 0), both by one unsigned minimum: the
+// smaller of d and d - slots (wrapping) is the slot when it lies below `slots`. Only other
+// keys — and tables of more than 2^30 slots, where a negative d could look like the next
+// range — divide.
 __device__ __forceinline__ int pht_slot(int key, int slots, int kmin) {
-  const int d = static_cast<int>(static_cast<unsigned>(key) - static_cast<unsigned>(kmin));
-  if (static_cast<unsigned>(d) < static_cast<unsigned>(slots)) return d;
-  if (static_cast<unsigned>(d) < 2u * static_cast<unsigned>(slots) && slots <= (1 << 30)) return d - slots;
-  return slow_mod(d, slots);
+  const unsigned d = static_cast<unsigned>(key) - static_cast<unsigned>(kmin), n = static_cast<unsigned>(slots);
+  const unsigned h = min(d, d - n);
+  if (h < n && n <= (1u << 30)) return static_cast<int>(h);
+  return slow_mod(static_cast<int>(d), slots);
 }
 
 // Longest a CTA waits on one bulk-copy stage before it gives up, sets

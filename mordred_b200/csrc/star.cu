@@ -264,10 +264,13 @@ int launch_star(const mb_star_args* a, cudaStream_t stream, int count32, const D
   // ---- calls with probes and no launch shape of their own -------------------------
   if (a->mirrors < 0 || a->mirrors > 2) return MB_ERR_ARG;
   if (a->pack < 0 || a->pack > 4) return MB_ERR_ARG;
+  // (segments shorter than the shape's default tile are refused below, as for every launch)
+  const TunedConfig tc = tuned_config(P.nf, a->num_probes, a->probe[0].layout, P.res_layout, P.total_val, P.n);
+  const int tile_of_defaults = tile_slices(tc.threads / 32) * 32 * tc.items;
   bool tiles = true;
   for (int c = 0; c < P.ncols; ++c) tiles = tiles && (P.gpu_cache != nullptr || aligned16(P.col[c]));
   if (P.np > 0 && a->agg_op != MB_AGG_MUL_PAYLOAD && tiles && P.n < (1ll << 32) &&
-      (P.gpu_cache == nullptr || P.seg_shift >= 8) && a->threads == 0 && a->items_per_thread == 0 && a->stages == 0 &&
+      (P.gpu_cache == nullptr || (1 << P.seg_shift) >= tile_of_defaults) && a->threads == 0 && a->items_per_thread == 0 && a->stages == 0 &&
       a->grid == 0 && a->mirrors != 2 && a->pack == 0 && a->group_mode != 1) {
     const int big = P.res_layout != MB_RES_SCALAR && P.total_val > 2048 ? 2 : 0;
     const int e = launch_ring(P, a->group_mode ? a->group_mode : big, *ds, stream);
@@ -276,7 +279,6 @@ int launch_star(const mb_star_args* a, cudaStream_t stream, int count32, const D
 
   // ---- launch configuration and shared-memory plan ------------------------------
   // Unset fields take the tuned configuration for this query shape (tuned_configs.h).
-  const TunedConfig tc = tuned_config(P.nf, a->num_probes, a->probe[0].layout, P.res_layout, P.total_val, P.n);
   const int threads = a->threads ? a->threads : tc.threads;
   const int items = a->items_per_thread ? a->items_per_thread : tc.items;
   if (threads % 32 != 0 || threads < 128 || threads > 768) return MB_ERR_ARG;

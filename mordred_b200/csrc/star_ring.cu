@@ -40,15 +40,21 @@ __host__ __device__ constexpr int ring_warp_bytes(int nst) {
   return static_cast<int>(sizeof(RingWarp)) + 2 * nst * kRingRows * 4;
 }
 
-// The word of slot h >= 0 of a table: 0 when absent, else nonzero; `payload` as probe_round's.
-__device__ __forceinline__ bool ring_lookup(const int* ht, int layout, int h, int& payload) {
-  if (layout == MB_HT_KEY) {
-    payload = 0;
-    return __ldg(ht + h) != 0;
-  }
-  const unsigned long long v = ldg_u64(ht + 2ll * h);
-  payload = layout == MB_HT_KEY_VAL ? static_cast<int>(v >> 32) : static_cast<int>(static_cast<unsigned>(v));
-  return v != 0ull;
+// The word of slot h >= 0 of a table, 0 when absent. Only the load: callers issue all of a
+// round's before they look at one.
+__device__ __forceinline__ unsigned long long ring_word(const int* ht, int layout, int h) {
+  unsigned long long v;
+  if (layout == MB_HT_KEY)
+    v = static_cast<unsigned>(__ldg(ht + h));
+  else
+    v = ldg_u64(ht + 2ll * h);
+  return v;
+}
+// The payload in a word, as probe_round's.
+__device__ __forceinline__ int ring_payload(int layout, unsigned long long v) {
+  return layout == MB_HT_KEY_VAL   ? static_cast<int>(v >> 32)
+         : layout == MB_HT_VAL_OFF ? static_cast<int>(static_cast<unsigned>(v))
+                                   : 0;
 }
 
 // Adds a row to the groups: `hh` its group index, val its value; keys written for the first
@@ -156,39 +162,45 @@ __global__ void __launch_bounds__(kRingMaxWarps * 32, 1) star_ring_kernel(const 
   const int nf = NFC >= 0 ? NFC : P.nf, nd = NDC >= 0 ? NDC : P.n_dense, ns = P.np - P.sparse_p0;
   const unsigned bias = static_cast<unsigned>(P.group_bias) + P.dense_bias;
   const bool two_cols = P.agg_op == MB_AGG_SUB || P.agg_op == MB_AGG_MUL;
-  const long long nslices = (P.n + kRingRows - 1) / kRingRows;
+  // the aggregate columns are gathered with the remaining keys, unless two or more tables can
+  // still drop the row: then only for the rows they leave
+  const bool early = (K ? ns - 1 - (nd - P.sparse_p0) : 0) <= 1;
+  // fewer than 2^32 rows: rows and slices count in 32 bits
+  const unsigned rows = static_cast<unsigned>(P.n);
+  const int nslices = static_cast<int>((P.n + kRingRows - 1) / kRingRows);
   // consecutive slices per CTA (its warps interleaved): a warp changes segment rarely
-  const long long per = (nslices + gridDim.x - 1) / gridDim.x;
-  const long long s_end = min(nslices, (blockIdx.x + 1) * per);
+  const int per = (nslices + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
+  const int s_end = min(nslices, (static_cast<int>(blockIdx.x) + 1) * per);
   const uint64_t policy = l2_policy_evict_first();
+  const uint32_t below = (1u << lane) - 1u;
   Accum A;
   bool failed = false;
 
   // lane c < nst copies staged column c: its column at the current segment
   const int* my_col = lane < nst ? P.col[P.r_col[lane]] : nullptr;
   const int* my_src = my_col;
-  long long cur_vseg = -1;
-  auto start = [&](long long s, int buf) {
-    const long long r0 = s * kRingRows;
-    long long at = r0;
+  int cur_vseg = -1;
+  auto start = [&](int s, int buf) {
+    const unsigned r0 = static_cast<unsigned>(s) * kRingRows;
+    unsigned at = r0;
     if (P.gpu_cache != nullptr) {
-      const long long vseg = r0 >> P.seg_shift;
+      const int vseg = static_cast<int>(r0 >> P.seg_shift);
       if (vseg != cur_vseg) {
         cur_vseg = vseg;
         const int seg = P.seg_group ? static_cast<int>(P.seg_group[vseg])
                                     : static_cast<int>((P.start_offset + r0) >> P.seg_shift);
         if (lane < nst) my_src = P.gpu_cache + (static_cast<long long>(__ldg(my_col + seg)) << P.seg_shift);
       }
-      at = r0 & ((1ll << P.seg_shift) - 1);
+      at = r0 & ((1u << P.seg_shift) - 1u);
     }
-    if (r0 + kRingRows <= P.n) {
+    if (rows - r0 >= kRingRows) {
       if (lane < nst) {
         fence_proxy_async_smem();
         mbar_arrive_expect_tx(&w.bar[buf], kRingRows * 4);
         bulk_g2s(stage + (buf * nst + lane) * kRingRows, my_src + at, kRingRows * 4, &w.bar[buf], policy);
       }
     } else {
-      const int have = static_cast<int>(P.n - r0);
+      const int have = static_cast<int>(rows - r0);
       for (int c = 0; c < nst; ++c) {
         const int* src = reinterpret_cast<const int*>(
             __shfl_sync(kFull, static_cast<unsigned long long>(reinterpret_cast<uintptr_t>(my_src)), c));
@@ -204,7 +216,7 @@ __global__ void __launch_bounds__(kRingMaxWarps * 32, 1) star_ring_kernel(const 
     mbar_fence_init();
   }
   __syncwarp();
-  long long s = blockIdx.x * per + warp;
+  int s = static_cast<int>(blockIdx.x) * per + warp;
   if (s < s_end) start(s, 0);
   if (s + nwarps < s_end) start(s + nwarps, 1);
   if (P.gmode == kGroupSmem) {
@@ -222,7 +234,7 @@ __global__ void __launch_bounds__(kRingMaxWarps * 32, 1) star_ring_kernel(const 
     const int* st = stage + buf * nst * kRingRows;
     int cnt = 0;
     if (!drain) {
-      const long long left = P.n - s * kRingRows;
+      const unsigned left = rows - static_cast<unsigned>(s) * kRingRows;
       uint32_t sel = (1u << kRingItems) - 1u;
       if (left >= kRingRows) {
         const bool ok = mbar_wait_bounded(&w.bar[buf], (it >> 1) & 1u);
@@ -231,7 +243,7 @@ __global__ void __launch_bounds__(kRingMaxWarps * 32, 1) star_ring_kernel(const 
         sel = 0;
 #pragma unroll
         for (int i = 0; i < kRingItems; ++i)
-          if (((i >> 2) * 32 + lane) * 4 + (i & 3) < left) sel |= 1u << i;
+          if (static_cast<unsigned>(((i >> 2) * 32 + lane) * 4 + (i & 3)) < left) sel |= 1u << i;
       }
       if (failed) sel = 0;
       // ---- dense part: bit j * 4 + e of the lane's mask is row (j * 32 + lane) * 4 + e ----
@@ -294,20 +306,13 @@ __global__ void __launch_bounds__(kRingMaxWarps * 32, 1) star_ring_kernel(const 
         }
         sel &= m;
       }
-      // ---- compaction: lane by lane, positions from a warp prefix sum ----
-      int incl = __popc(sel);
-      const int own = incl;
+      // ---- compaction: a ballot per item gives the survivors' places ----
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(kFull, incl, o);
-        if (lane >= o) incl += y;
-      }
-      cnt = __shfl_sync(kFull, incl, 31);
-      uint16_t* to = w.off + (incl - own);
-      while (sel) {
-        const int i = __ffs(sel) - 1;
-        sel &= sel - 1;
-        *to++ = static_cast<uint16_t>((i >> 2) * 128 + lane * 4 + (i & 3));
+      for (int i = 0; i < kRingItems; ++i) {
+        const bool on = (sel >> i) & 1u;
+        const uint32_t b = __ballot_sync(kFull, on);
+        if (on) w.off[cnt + __popc(b & below)] = static_cast<uint16_t>((i >> 2) * 128 + lane * 4 + (i & 3));
+        cnt += __popc(b);
       }
       __syncwarp();
     }
@@ -344,20 +349,27 @@ __global__ void __launch_bounds__(kRingMaxWarps * 32, 1) star_ring_kernel(const 
             }
             if (!ok[r]) h[r] = 0;
           }
-          bool in[2];
+          unsigned long long word[2];
+          if (layout == MB_HT_KEY) {
+            word[0] = ring_word(ht, MB_HT_KEY, h[0]);
+            word[1] = ring_word(ht, MB_HT_KEY, h[1]);
+          } else {
+            word[0] = ring_word(ht, MB_HT_KEY_VAL, h[0]);
+            word[1] = ring_word(ht, MB_HT_KEY_VAL, h[1]);
+          }
 #pragma unroll
-          for (int r = 0; r < 2; ++r) in[r] = ring_lookup(ht, layout, h[r], pay[r]);
-#pragma unroll
-          for (int r = 0; r < 2; ++r) ok[r] = ok[r] && in[r];
+          for (int r = 0; r < 2; ++r) {
+            ok[r] = ok[r] && word[r] != 0ull;
+            pay[r] = ring_payload(layout, word[r]);
+          }
         }
       }
       const uint32_t b0 = __ballot_sync(kFull, ok[0]), b1 = __ballot_sync(kFull, ok[1]);
       const int add = __popc(b0) + __popc(b1);
-      const uint32_t below = (1u << lane) - 1u;
       bool pushed = add == 0;
       while (true) {
         if (!pushed && held + add <= kRingCap) {
-          const int r0 = static_cast<int>(s * kRingRows);  // rows of the call, as 32 bits
+          const int r0 = s * kRingRows;
           if (ok[0]) w.ring[held + __popc(b0 & below)] = make_int2(pay[0], r0 + row[0]);
           if (ok[1]) w.ring[held + __popc(b0) + __popc(b1 & below)] = make_int2(pay[1], r0 + row[1]);
           held += add;
@@ -376,47 +388,81 @@ __global__ void __launch_bounds__(kRingMaxWarps * 32, 1) star_ring_kernel(const 
         for (int q = 0; q < MB_MAX_PROBES; ++q) gv[q] = 0;
         if (K) gv[0] = entry.x;
         constexpr int kQ0 = K ? 1 : 0;
+        int seg = 0;
+        const int* in_seg = nullptr;
         if (P.gpu_cache == nullptr) {
 #pragma unroll
           for (int q = kQ0; q < MB_MAX_PROBES; ++q)
             if (q < ns) gv[q] = __ldg(P.col[P.p_col[P.sp_ord[q]]] + r);
-          a0 = __ldg(P.col[P.a_col[0]] + r);
-          if (two_cols) a1 = __ldg(P.col[P.a_col[1]] + r);
+          if (early) {
+            a0 = __ldg(P.col[P.a_col[0]] + r);
+            if (two_cols) a1 = __ldg(P.col[P.a_col[1]] + r);
+          }
         } else {
           const long long vseg = r >> P.seg_shift;
-          const int seg = P.seg_group ? static_cast<int>(P.seg_group[vseg])
+          seg = P.seg_group ? static_cast<int>(P.seg_group[vseg])
                                       : static_cast<int>((P.start_offset + r) >> P.seg_shift);
-          const int* in_seg = P.gpu_cache + (r & ((1ll << P.seg_shift) - 1));
+          in_seg = P.gpu_cache + (r & ((1ll << P.seg_shift) - 1));
 #pragma unroll
           for (int q = kQ0; q < MB_MAX_PROBES; ++q)
             if (q < ns) gv[q] = __ldg(P.col[P.p_col[P.sp_ord[q]]] + seg);
-          a0 = __ldg(P.col[P.a_col[0]] + seg);
-          if (two_cols) a1 = __ldg(P.col[P.a_col[1]] + seg);
+          if (early) {
+            a0 = __ldg(P.col[P.a_col[0]] + seg);
+            if (two_cols) a1 = __ldg(P.col[P.a_col[1]] + seg);
+          }
 #pragma unroll
           for (int q = kQ0; q < MB_MAX_PROBES; ++q)
             if (q < ns) gv[q] = __ldg(in_seg + (static_cast<long long>(gv[q]) << P.seg_shift));
-          a0 = __ldg(in_seg + (static_cast<long long>(a0) << P.seg_shift));
-          if (two_cols) a1 = __ldg(in_seg + (static_cast<long long>(a1) << P.seg_shift));
+          if (early) {
+            a0 = __ldg(in_seg + (static_cast<long long>(a0) << P.seg_shift));
+            if (two_cols) a1 = __ldg(in_seg + (static_cast<long long>(a1) << P.seg_shift));
+          }
         }
-        bool in[MB_MAX_PROBES], below_min[MB_MAX_PROBES];
+        unsigned long long word[MB_MAX_PROBES];
+        bool below_min[MB_MAX_PROBES];
 #pragma unroll
         for (int q = kQ0; q < MB_MAX_PROBES; ++q) {
-          in[q] = true;
+          word[q] = 1ull;
           below_min[q] = false;
-          if (q >= ns) continue;
-          const int p = P.sp_ord[q];
-          const int h = pht_slot(gv[q], P.p_slots[p], P.p_kmin[p]);
-          below_min[q] = h < 0;
-          in[q] = ring_lookup(P.p_ht[p], P.p_layout[p], h < 0 ? 0 : h, gv[q]);
+          if (q < ns) {
+            const int p = P.sp_ord[q];
+            int h = pht_slot(gv[q], P.p_slots[p], P.p_kmin[p]);
+            below_min[q] = h < 0;
+            h = max(h, 0);
+            // two loads under opposite predicates, so that the probes share one basic block
+            const int* ht = P.p_ht[p];
+            const bool key = P.p_layout[p] == MB_HT_KEY;
+            unsigned lo = 0, hi = 0;
+            asm volatile(
+                "{\n\t.reg .pred k;\n\t"
+                "setp.ne.u32 k, %4, 0;\n\t"
+                "@k ld.global.nc.u32 %0, [%2];\n\t"
+                "@!k ld.global.nc.v2.u32 {%0, %1}, [%3];\n\t}"
+                : "+r"(lo), "+r"(hi)
+                : "l"(ht + h), "l"(ht + 2ll * h), "r"(key ? 1u : 0u));
+            word[q] = (static_cast<unsigned long long>(hi) << 32) | lo;
+          }
         }
 #pragma unroll
         for (int q = kQ0; q < MB_MAX_PROBES; ++q) {
           if (q >= ns) continue;
           if (live && below_min[q]) A.bad_probe = true;
-          live = live && !below_min[q] && in[q];
+          live = live && !below_min[q] && word[q] != 0ull;
+          gv[q] = ring_payload(P.p_layout[P.sp_ord[q]], word[q]);
         }
         if (live) {
           if (P.count_after < 0) ++A.cnt;
+          if (!early) {
+            if (P.gpu_cache == nullptr) {
+              a0 = __ldg(P.col[P.a_col[0]] + r);
+              if (two_cols) a1 = __ldg(P.col[P.a_col[1]] + r);
+            } else {
+              a0 = __ldg(P.col[P.a_col[0]] + seg);
+              if (two_cols) a1 = __ldg(P.col[P.a_col[1]] + seg);
+              a0 = __ldg(in_seg + (static_cast<long long>(a0) << P.seg_shift));
+              if (two_cols) a1 = __ldg(in_seg + (static_cast<long long>(a1) << P.seg_shift));
+            }
+          }
           const unsigned u0 = static_cast<unsigned>(a0), u1 = static_cast<unsigned>(a1);
           const int val = static_cast<int>(P.agg_op == MB_AGG_SUM ? u0 : P.agg_op == MB_AGG_SUB ? u0 - u1 : u0 * u1);
           if (P.gmode == kGroupScalar) {
