@@ -170,6 +170,23 @@ int mb_build_pht(const int* filter_col, int filter_mode, int c1, int c2,
                  int* ht, int num_slots, int key_min, uint32_t* presence,
                  mb_stream_t stream);
 
+/* The tables of a query in two launches: clears every table (int[num_slots], with dim_val
+ * int[2 * num_slots]), its presence bitmap and `zero` (zero_words 32-bit words, optional: the
+ * query's result), then builds each as mb_build_pht does. */
+#define MB_MAX_TABLE_BUILDS 8
+typedef struct mb_table_build {
+  const int* filter_col;
+  int filter_mode, c1, c2;
+  const int* dim_key;
+  const int* dim_val;
+  int num_tuples;
+  int* ht;
+  int num_slots, key_min;
+  uint32_t* presence;
+} mb_table_build;
+int mb_build_tables(const mb_table_build* builds, int num_builds, int* zero, int64_t zero_words,
+                    mb_stream_t stream);
+
 /* Unfiltered PHT_2 build: src/ops/join.cu:21-40 build_kernel. */
 int mb_join_build(const int* dim_key, const int* dim_val, int num_tuples,
                   int* hash_table, int num_slots, mb_stream_t stream);

@@ -85,6 +85,12 @@ class MbBuildArgsGPU(C.Structure):
                 ("val_min", C.c_int), ("val_max", C.c_int)]
 
 
+class MbTableBuild(C.Structure):
+    _fields_ = [("filter_col", C.c_void_p), ("filter_mode", C.c_int), ("c1", C.c_int), ("c2", C.c_int),
+                ("dim_key", C.c_void_p), ("dim_val", C.c_void_p), ("num_tuples", C.c_int), ("ht", C.c_void_p),
+                ("num_slots", C.c_int), ("key_min", C.c_int), ("presence", C.c_void_p)]
+
+
 P = C.c_void_p
 I = C.c_int
 I64 = C.c_int64
@@ -95,6 +101,7 @@ PS = C.POINTER
 SIGNATURES = {
     "mb_star_query": (I, [PS(MbStarArgs), P]),
     "mb_build_pht": (I, [P, I, I, I, P, P, I, P, I, I, P, P]),
+    "mb_build_tables": (I, [PS(MbTableBuild), I, P, I64, P]),
     "mb_join_build": (I, [P, P, I, P, I, P]),
     "mb_join_probe": (I, [P, P, I, P, I, P, P]),
     "mb_q11_query": (I, [P, P, P, P, I, P, P, P]),

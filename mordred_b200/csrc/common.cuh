@@ -128,6 +128,13 @@ __device__ __forceinline__ void smem_add_i64(unsigned long long* sum, int v) {
   if (hi != 0u) atomicAdd(w + 1, hi);
 }
 
+// Programmatic dependent launch: a kernel launched with launch_dependent() may be set up while
+// its predecessor in the stream still runs, and waits here — before it touches global memory —
+// until the predecessor has completed and its writes are visible. Short kernels let their
+// successor be set up from the start (allow_dependent).
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void allow_dependent() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ void set_status(unsigned int* status, unsigned int bits) {
   if (status) atomicOr(status, bits);
 }
@@ -149,6 +156,24 @@ struct DeviceState {
 // Returns nullptr (and sets *err) if the current device cannot be initialised.
 DeviceState* current_device_state(int* err);
 void note_launches(unsigned long long n);
+
+// Launch `fn` on `stream` so that its set-up overlaps the end of the kernel before it; `fn`
+// begins with wait_for_predecessor().
+template <class... Params, class... Args>
+inline cudaError_t launch_dependent(void (*fn)(Params...), int grid, int block, size_t smem, cudaStream_t stream,
+                                    Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(static_cast<unsigned>(block));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, fn, static_cast<Params>(args)...);
+}
 
 inline int cuda_status(cudaError_t e) { return e == cudaSuccess ? MB_OK : MB_ERR_CUDA; }
 

@@ -210,6 +210,7 @@ __global__ void __launch_bounds__(kRingMaxWarps * 32, 1) star_ring_kernel(const 
     }
   };
 
+  wait_for_predecessor();
   if (lane == 0) {
     mbar_init(&w.bar[0], nst);
     mbar_init(&w.bar[1], nst);
@@ -612,8 +613,9 @@ int launch_ring(StarPlan& P, int group_mode, const DeviceState& ds, cudaStream_t
   if (warps > per && per >= 16) warps = static_cast<int>(per);
   P.smem_total = off + warps * ring_warp_bytes(P.r_nst);
   const KernelFn fn = kRing[P.nf > 0 ? 1 : 0][P.n_dense > 1 ? 2 : P.n_dense][key ? 1 : 0];
-  fn<<<static_cast<int>(blocks), warps * 32, P.smem_total, stream>>>(P);
-  if (cudaGetLastError() != cudaSuccess) return MB_ERR_LAUNCH;
+  if (launch_dependent(fn, static_cast<int>(blocks), warps * 32, static_cast<size_t>(P.smem_total), stream, P) !=
+      cudaSuccess)
+    return MB_ERR_LAUNCH;
   note_launches(1);
   return MB_OK;
 }

@@ -196,16 +196,23 @@ def query_a(t: dict, ws: StarWorkspace, category: int = 1, region: int = 1, stre
     return probe_a(t, ws, stream)
 
 
+def build_tables(builds: list[tuple], zero=None, stream=None) -> None:
+    """Clear and build a query's hash tables in two launches (mb_build_tables). A build is
+    (filter column, mode, c1, c2, key column, payload column, rows, table, slots, key_min);
+    `zero` is cleared with them (the query's result)."""
+    arr = (L.MbTableBuild * len(builds))(*[(_p(f), mode, c1, c2, _p(key), _p(val), n, _p(ht), slots, kmin, None)
+                                           for f, mode, c1, c2, key, val, n, ht, slots, kmin in builds])
+    L.call("mb_build_tables", arr, len(builds), _p(zero), 0 if zero is None else zero.numel() * zero.element_size() // 4,
+           _stream(stream))
+
+
 def build_a(t: dict, ws: StarWorkspace, category: int = 1, region: int = 1, stream=None) -> None:
-    s, st = ws.sizes, _stream(stream)
-    for k in ("ht_s", "ht_p_a", "ht_d", "res_a"):
-        ws[k].zero_()
-    L.call("mb_build_pht", _p(t["s_region"]), L.MB_FILTER_EQ, region, 0, _p(t["s_suppkey"]), None,
-           s.s_len, _p(ws["ht_s"]), s.s_len, 0, None, st)
-    L.call("mb_build_pht", _p(t["p_category"]), L.MB_FILTER_EQ, category, 0, _p(t["p_partkey"]),
-           _p(t["p_brand1"]), s.p_len, _p(ws["ht_p_a"]), s.p_len, 0, None, st)
-    L.call("mb_build_pht", None, 0, 0, 0, _p(t["d_datekey"]), _p(t["d_year"]), s.d_len,
-           _p(ws["ht_d"]), ws.date_slots, DATE_MIN, None, st)
+    s, eq = ws.sizes, L.MB_FILTER_EQ
+    build_tables([
+        (t["s_region"], eq, region, 0, t["s_suppkey"], None, s.s_len, ws["ht_s"], s.s_len, 0),
+        (t["p_category"], eq, category, 0, t["p_partkey"], t["p_brand1"], s.p_len, ws["ht_p_a"], s.p_len, 0),
+        (None, 0, 0, 0, t["d_datekey"], t["d_year"], s.d_len, ws["ht_d"], ws.date_slots, DATE_MIN)],
+        ws["res_a"], stream)
 
 
 def probe_a(t: dict, ws: StarWorkspace, stream=None) -> torch.Tensor:
@@ -225,17 +232,13 @@ def query_b(t: dict, ws: StarWorkspace, c_region: int = 1, s_region: int = 1, mf
 
 def build_b(t: dict, ws: StarWorkspace, c_region: int = 1, s_region: int = 1, mfgr=(0, 1),
             stream=None) -> None:
-    s, st = ws.sizes, _stream(stream)
-    for k in ("ht_s", "ht_c", "ht_p_b", "ht_d", "res_b"):
-        ws[k].zero_()
-    L.call("mb_build_pht", _p(t["s_region"]), L.MB_FILTER_EQ, s_region, 0, _p(t["s_suppkey"]), None,
-           s.s_len, _p(ws["ht_s"]), s.s_len, 0, None, st)
-    L.call("mb_build_pht", _p(t["c_region"]), L.MB_FILTER_EQ, c_region, 0, _p(t["c_custkey"]),
-           _p(t["c_nation"]), s.c_len, _p(ws["ht_c"]), s.c_len, 0, None, st)
-    L.call("mb_build_pht", _p(t["p_mfgr"]), L.MB_FILTER_EQ_OR_EQ, mfgr[0], mfgr[1], _p(t["p_partkey"]),
-           None, s.p_len, _p(ws["ht_p_b"]), s.p_len, 0, None, st)
-    L.call("mb_build_pht", None, 0, 0, 0, _p(t["d_datekey"]), _p(t["d_year"]), s.d_len,
-           _p(ws["ht_d"]), ws.date_slots, DATE_MIN, None, st)
+    s, eq = ws.sizes, L.MB_FILTER_EQ
+    build_tables([
+        (t["s_region"], eq, s_region, 0, t["s_suppkey"], None, s.s_len, ws["ht_s"], s.s_len, 0),
+        (t["c_region"], eq, c_region, 0, t["c_custkey"], t["c_nation"], s.c_len, ws["ht_c"], s.c_len, 0),
+        (t["p_mfgr"], L.MB_FILTER_EQ_OR_EQ, mfgr[0], mfgr[1], t["p_partkey"], None, s.p_len, ws["ht_p_b"], s.p_len, 0),
+        (None, 0, 0, 0, t["d_datekey"], t["d_year"], s.d_len, ws["ht_d"], ws.date_slots, DATE_MIN)],
+        ws["res_b"], stream)
 
 
 def probe_b(t: dict, ws: StarWorkspace, stream=None) -> torch.Tensor:
