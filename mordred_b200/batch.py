@@ -311,7 +311,7 @@ class AloneWorkspace:
 
 def run_alone(t: dict, ws: AloneWorkspace, q: Query, res: torch.Tensor, n_rows: int, stream=None) -> None:
     """One query the reference's way: filtered PHT builds, then the fused probe."""
-    s, st = ws.sizes, ssb._stream(stream)
+    s = ws.sizes
     B = L.MB_FILTER_BETWEEN
     date = dict(col=t["lo_orderdate"], mode=B, c1=q.date[0], c2=q.date[1])
     if q.template == "agg":
@@ -323,30 +323,25 @@ def run_alone(t: dict, ws: AloneWorkspace, q: Query, res: torch.Tensor, n_rows: 
                              res_layout=L.MB_RES_SCALAR, res=res)
         ssb.star_query(args, stream)
         return
-    ws.ht_s.zero_()
-    ws.ht_d.zero_()
-    L.call("mb_build_pht", ssb._p(t["s_region"]), B, q.s_region[0], q.s_region[1], ssb._p(t["s_suppkey"]), None,
-           s.s_len, ssb._p(ws.ht_s), s.s_len, 0, None, st)
-    L.call("mb_build_pht", None, 0, 0, 0, ssb._p(t["d_datekey"]), ssb._p(t["d_year"]), s.d_len, ssb._p(ws.ht_d),
-           ssb.DATE_SLOTS, ssb.DATE_MIN, None, st)
+    builds = [(t["s_region"], B, q.s_region[0], q.s_region[1], t["s_suppkey"], None, s.s_len, ws.ht_s, s.s_len, 0),
+              (None, 0, 0, 0, t["d_datekey"], t["d_year"], s.d_len, ws.ht_d, ssb.DATE_SLOTS, ssb.DATE_MIN)]
+    if q.template == "qa":
+        builds.append((t["p_category"], B, q.category[0], q.category[1], t["p_partkey"], t["p_brand1"], s.p_len, ws.ht_p,
+                       s.p_len, 0))
+    else:
+        builds += [(t["c_region"], B, q.c_region[0], q.c_region[1], t["c_custkey"], t["c_nation"], s.c_len, ws.ht_c,
+                    s.c_len, 0),
+                   (t["p_mfgr"], B, q.mfgr[0], q.mfgr[1], t["p_partkey"], None, s.p_len, ws.ht_pk, s.p_len, 0)]
+    ssb.build_tables(builds, stream=stream)
     d_probe = dict(fkey=t["lo_orderdate"], ht=ws.ht_d, num_slots=ssb.DATE_SLOTS, key_min=ssb.DATE_MIN,
                    layout=L.MB_HT_KEY_VAL, min_val=1992, unique_val=1, res_slot=0)
     s_probe = dict(fkey=t["lo_suppkey"], ht=ws.ht_s, num_slots=s.s_len, layout=L.MB_HT_KEY)
     if q.template == "qa":
-        ws.ht_p.zero_()
-        L.call("mb_build_pht", ssb._p(t["p_category"]), B, q.category[0], q.category[1], ssb._p(t["p_partkey"]),
-               ssb._p(t["p_brand1"]), s.p_len, ssb._p(ws.ht_p), s.p_len, 0, None, st)
         probes = [s_probe, dict(fkey=t["lo_partkey"], ht=ws.ht_p, num_slots=s.p_len, layout=L.MB_HT_KEY_VAL,
                                 unique_val=7, res_slot=1), d_probe]
         args = ssb.star_args(num_rows=n_rows, filters=[date], probes=probes, aggr=[t["lo_revenue"]],
                              agg_op=L.MB_AGG_SUM, total_val=ssb.QA_GROUPS, res_layout=L.MB_RES_CRYSTAL4, res=res)
     else:
-        ws.ht_c.zero_()
-        ws.ht_pk.zero_()
-        L.call("mb_build_pht", ssb._p(t["c_region"]), B, q.c_region[0], q.c_region[1], ssb._p(t["c_custkey"]),
-               ssb._p(t["c_nation"]), s.c_len, ssb._p(ws.ht_c), s.c_len, 0, None, st)
-        L.call("mb_build_pht", ssb._p(t["p_mfgr"]), B, q.mfgr[0], q.mfgr[1], ssb._p(t["p_partkey"]), None, s.p_len,
-               ssb._p(ws.ht_pk), s.p_len, 0, None, st)
         probes = [s_probe, dict(fkey=t["lo_custkey"], ht=ws.ht_c, num_slots=s.c_len, layout=L.MB_HT_KEY_VAL,
                                 unique_val=7, res_slot=1),
                   dict(fkey=t["lo_partkey"], ht=ws.ht_pk, num_slots=s.p_len, layout=L.MB_HT_KEY), d_probe]

@@ -388,6 +388,7 @@ __global__ void __launch_bounds__((NCW + 1) * 32, 1) batch_kernel(const __grid_c
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int S = P.stages;
 
+  wait_for_predecessor();  // the mask kernel, or the batch before
   // ---- set-up: accumulators, descriptors, masks, small tables, barriers ------------
   {
     unsigned long long* s_acc = reinterpret_cast<unsigned long long*>(smem + P.smem_acc_off);
@@ -785,6 +786,8 @@ __global__ void __launch_bounds__((NCW + 1) * 32, 1) batch_kernel(const __grid_c
 // (256 queries: 8 us; each thread walking all queries' descriptors: 70 us).
 __global__ void batch_mask_kernel(const __grid_constant__ BatchPlan P, int tasks) {
   const int lane = threadIdx.x & 31;
+  allow_dependent();
+  wait_for_predecessor();
   for (int task = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; task < tasks; task += (gridDim.x * blockDim.x) >> 5) {
     int rest = task, first = 0, last = 0;  // the table's attributes
     for (;; first = last + 1) {
@@ -1447,8 +1450,9 @@ extern "C" int mb_batch_run(const mb_batch_args* a, mb_stream_t stream) {
     for (int f = 0; f < P.nfields; ++f) tasks += P.at[f].last ? (P.at[f].ent + 31) / 32 * P.nwords : 0;
     long long blocks = (tasks + 3) / 4;
     if (blocks > ds->num_sms * 8) blocks = ds->num_sms * 8;
-    batch_mask_kernel<<<static_cast<int>(blocks), 128, 0, st>>>(P, static_cast<int>(tasks));
-    if (cudaGetLastError() != cudaSuccess) return MB_ERR_LAUNCH;
+    if (launch_dependent(batch_mask_kernel, static_cast<int>(blocks), 128, 0, st, P, static_cast<int>(tasks)) !=
+        cudaSuccess)
+      return MB_ERR_LAUNCH;
     note_launches(1);
   }
   int grid = a->grid;
@@ -1463,8 +1467,8 @@ extern "C" int mb_batch_run(const mb_batch_args* a, mb_stream_t stream) {
   long long want = P.nfull > 0 ? P.nfull : (P.n + threads - 1) / threads;
   if (want < 1) want = 1;
   if (grid > want) grid = static_cast<int>(want);
-  var->fn<<<grid, threads + 32, smem, st>>>(P);
-  if (cudaGetLastError() != cudaSuccess) return MB_ERR_LAUNCH;
+  if (launch_dependent(var->fn, grid, threads + 32, static_cast<size_t>(smem), st, P) != cudaSuccess)
+    return MB_ERR_LAUNCH;
   note_launches(1);
   return MB_OK;
 }

@@ -189,6 +189,7 @@ __global__ void __launch_bounds__(kSelMaxWarps * 32, 1) select_slices_kernel(con
     }
   };
 
+  wait_for_predecessor();
   if (lane == 0) {
     mbar_init(&w.bar, 1);
     mbar_fence_init();
@@ -551,8 +552,9 @@ static int launch_slices(SelPlan& P, const DeviceState& ds, cudaStream_t st) {
   if (warps > kSelMaxWarps) warps = kSelMaxWarps;
   if (warps > per && per >= 16) warps = static_cast<int>(per);
   const int smem = warps * warp_bytes(nc) + 4 * P.bm_words;
-  kSlices[P.nf][2 * (bm ? 1 : 0) + (key ? 1 : 0)]<<<static_cast<int>(blocks), warps * 32, smem, st>>>(P);
-  if (cudaGetLastError() != cudaSuccess) return MB_ERR_LAUNCH;
+  if (launch_dependent(kSlices[P.nf][2 * (bm ? 1 : 0) + (key ? 1 : 0)], static_cast<int>(blocks), warps * 32,
+                       static_cast<size_t>(smem), st, P) != cudaSuccess)
+    return MB_ERR_LAUNCH;
   note_launches(1);
   return MB_OK;
 }

@@ -91,6 +91,7 @@ __global__ void __launch_bounds__(kListThreads, kListCtas) list_kernel(const __g
   unsigned long long* s_sum = reinterpret_cast<unsigned long long*>(lsmem);
   uint32_t* s_touch = reinterpret_cast<uint32_t*>(lsmem + 8 * P.total_val);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  wait_for_predecessor();
   if (P.gmode == kGroupSmem) {
     for (int g = tid; g < P.total_val; g += kListThreads) s_sum[g] = 0;
     for (int w = tid; w < (P.total_val + 31) / 32; w += kListThreads) s_touch[w] = 0;
@@ -403,8 +404,8 @@ int launch_list(const mb_star_args* a, cudaStream_t stream, const DeviceState* d
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
   const auto fn = P.gpu_cache != nullptr ? list_kernel<true> : list_kernel<false>;
-  fn<<<static_cast<int>(blocks), kListThreads, smem, stream>>>(P);
-  if (cudaGetLastError() != cudaSuccess) return MB_ERR_LAUNCH;
+  if (launch_dependent(fn, static_cast<int>(blocks), kListThreads, static_cast<size_t>(smem), stream, P) != cudaSuccess)
+    return MB_ERR_LAUNCH;
   note_launches(1);
   return MB_OK;
 }

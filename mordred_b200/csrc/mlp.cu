@@ -137,6 +137,7 @@ __global__ void __launch_bounds__(kFwdWarps * 32, 1) mlp_forward_kernel(const fl
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
+  wait_for_predecessor();
   long long tile = blockIdx.x + static_cast<long long>(gridDim.x) * warp;
   for (int i = lane; i < kTile * kFwdXRow; i += 32) xs[i] = 0.f;
   __syncwarp();
@@ -268,6 +269,8 @@ __global__ void __launch_bounds__(kBwdThreads) mlp_backward_kernel(const float* 
   constexpr int kWarps = kBwdThreads / 32;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int j = tid & (kHid - 1), b0 = (tid >> 6) * NS;
+  allow_dependent();
+  wait_for_predecessor();
 #pragma unroll
   for (int i = 0; i < kIn * kHid / kBwdThreads; ++i) s.w1[i * kBwdThreads + tid] = params[kW1 + i * kBwdThreads + tid];
 #pragma unroll
@@ -407,6 +410,8 @@ __global__ void __launch_bounds__(kBwdThreads) mlp_backward_kernel(const float* 
 __global__ void mlp_adam_kernel(float* __restrict__ params, const float* __restrict__ grads, float* __restrict__ m,
                                 float* __restrict__ v, int n, float lr, float beta1, float beta2, float eps,
                                 float bc1, float bc2, float weight_decay) {
+  allow_dependent();
+  wait_for_predecessor();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float g = grads[i] + weight_decay * params[i];
     const float mi = beta1 * m[i] + (1.f - beta1) * g;
@@ -454,11 +459,9 @@ extern "C" int mb_mlp_forward(const float* params, const float* x, int batch, fl
   const int tile = 8 * (small ? kFwdSmall : kFwdLarge);
   const long long tiles = (static_cast<long long>(batch) + tile - 1) / tile;
   const int grid = static_cast<int>(tiles < ds->num_sms ? tiles : ds->num_sms);
-  if (small)
-    mlp_forward_kernel<kFwdSmall><<<grid, kFwdWarps * 32, sizeof(FwdSmem<kFwdSmall>), st>>>(params, x, batch, y);
-  else
-    mlp_forward_kernel<kFwdLarge><<<grid, kFwdWarps * 32, sizeof(FwdSmem<kFwdLarge>), st>>>(params, x, batch, y);
-  if (cudaGetLastError() != cudaSuccess) return MB_ERR_LAUNCH;
+  const auto fn = small ? mlp_forward_kernel<kFwdSmall> : mlp_forward_kernel<kFwdLarge>;
+  const size_t smem = small ? sizeof(FwdSmem<kFwdSmall>) : sizeof(FwdSmem<kFwdLarge>);
+  if (launch_dependent(fn, grid, kFwdWarps * 32, smem, st, params, x, batch, y) != cudaSuccess) return MB_ERR_LAUNCH;
   note_launches(1);
   return MB_OK;
 }
@@ -475,13 +478,10 @@ extern "C" int mb_mlp_backward(const float* params, const float* x, const float*
   const int tile = small ? kBwdSmall : kBwdLarge;
   const long long tiles = (static_cast<long long>(batch) + tile - 1) / tile;
   const int grid = static_cast<int>(tiles < ds->num_sms ? tiles : ds->num_sms);
-  if (small)
-    mlp_backward_kernel<kBwdSmall><<<grid, kBwdThreads, sizeof(BwdSmem<kBwdSmall>), st>>>(params, x, target, batch,
-                                                                                         grads, loss_sum);
-  else
-    mlp_backward_kernel<kBwdLarge><<<grid, kBwdThreads, sizeof(BwdSmem<kBwdLarge>), st>>>(params, x, target, batch,
-                                                                                         grads, loss_sum);
-  if (cudaGetLastError() != cudaSuccess) return MB_ERR_LAUNCH;
+  const auto fn = small ? mlp_backward_kernel<kBwdSmall> : mlp_backward_kernel<kBwdLarge>;
+  const size_t smem = small ? sizeof(BwdSmem<kBwdSmall>) : sizeof(BwdSmem<kBwdLarge>);
+  if (launch_dependent(fn, grid, kBwdThreads, smem, st, params, x, target, batch, grads, loss_sum) != cudaSuccess)
+    return MB_ERR_LAUNCH;
   note_launches(1);
   return MB_OK;
 }
@@ -495,9 +495,9 @@ extern "C" int mb_mlp_adam(float* params, const float* grads, float* m, float* v
   const float bc2 = static_cast<float>(1.0 - std::pow(static_cast<double>(beta2), step));
   int blocks = (n + 255) / 256;
   if (blocks > 1024) blocks = 1024;
-  mlp_adam_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(params, grads, m, v, n, lr, beta1, beta2,
-                                                                         eps, bc1, bc2, weight_decay);
-  if (cudaGetLastError() != cudaSuccess) return MB_ERR_LAUNCH;
+  if (launch_dependent(mlp_adam_kernel, blocks, 256, 0, static_cast<cudaStream_t>(stream), params, grads, m, v, n, lr,
+                       beta1, beta2, eps, bc1, bc2, weight_decay) != cudaSuccess)
+    return MB_ERR_LAUNCH;
   note_launches(1);
   return MB_OK;
 }

@@ -407,8 +407,8 @@ int launch_star(const mb_star_args* a, cudaStream_t stream, int count32, const D
   }
   if (grid > want) grid = static_cast<int>(want);
 
-  var->fn<<<grid, threads + 32, smem, stream>>>(P);
-  if (cudaGetLastError() != cudaSuccess) return MB_ERR_LAUNCH;
+  if (launch_dependent(var->fn, grid, threads + 32, static_cast<size_t>(smem), stream, P) != cudaSuccess)
+    return MB_ERR_LAUNCH;
   note_launches(1);
   return MB_OK;
 }

@@ -777,6 +777,7 @@ __global__ void __launch_bounds__((NCW + 1) * 32, star_min_ctas(NCW)) star_kerne
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int S = P.stages;
 
+  wait_for_predecessor();
   // ---- set-up: group accumulators, staged presence bitmaps, barriers ----------
   if (P.gmode == kGroupSmem) {
     for (int g = tid; g < P.total_val; g += NWARPS * 32) s_sum[g] = 0;

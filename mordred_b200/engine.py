@@ -296,25 +296,17 @@ class Executor(CpuShare):
     def build_gpu(self, q: B.Query) -> None:
         if q.template == "agg":
             return
-        d, s, st = self.t.dims, self.t.sizes, ssb._stream()
+        d, s, ht = self.t.dims, self.t.sizes, self.ht
         BT = L.MB_FILTER_BETWEEN
-        self.ht["s"].zero_()
-        self.ht["d"].zero_()
-        L.call("mb_build_pht", ssb._p(d["s_region"]), BT, q.s_region[0], q.s_region[1], ssb._p(d["s_suppkey"]), None,
-               s.s_len, ssb._p(self.ht["s"]), s.s_len, 0, None, st)
-        L.call("mb_build_pht", None, 0, 0, 0, ssb._p(d["d_datekey"]), ssb._p(d["d_year"]), s.d_len,
-               ssb._p(self.ht["d"]), ssb.DATE_SLOTS, ssb.DATE_MIN, None, st)
+        builds = [(d["s_region"], BT, *q.s_region, d["s_suppkey"], None, s.s_len, ht["s"], s.s_len, 0),
+                  (None, 0, 0, 0, d["d_datekey"], d["d_year"], s.d_len, ht["d"], ssb.DATE_SLOTS, ssb.DATE_MIN)]
         if q.template == "qa":
-            self.ht["p_kv"].zero_()
-            L.call("mb_build_pht", ssb._p(d["p_category"]), BT, q.category[0], q.category[1], ssb._p(d["p_partkey"]),
-                   ssb._p(d["p_brand1"]), s.p_len, ssb._p(self.ht["p_kv"]), s.p_len, 0, None, st)
+            builds.append((d["p_category"], BT, *q.category, d["p_partkey"], d["p_brand1"], s.p_len, ht["p_kv"], s.p_len,
+                           0))
         else:
-            self.ht["c"].zero_()
-            self.ht["p_key"].zero_()
-            L.call("mb_build_pht", ssb._p(d["c_region"]), BT, q.c_region[0], q.c_region[1], ssb._p(d["c_custkey"]),
-                   ssb._p(d["c_nation"]), s.c_len, ssb._p(self.ht["c"]), s.c_len, 0, None, st)
-            L.call("mb_build_pht", ssb._p(d["p_mfgr"]), BT, q.mfgr[0], q.mfgr[1], ssb._p(d["p_partkey"]), None,
-                   s.p_len, ssb._p(self.ht["p_key"]), s.p_len, 0, None, st)
+            builds += [(d["c_region"], BT, *q.c_region, d["c_custkey"], d["c_nation"], s.c_len, ht["c"], s.c_len, 0),
+                       (d["p_mfgr"], BT, *q.mfgr, d["p_partkey"], None, s.p_len, ht["p_key"], s.p_len, 0)]
+        ssb.build_tables(builds)
 
     def _launch_wave(self, q: B.Query, segs: list[int], w: int) -> None:
         segs = self._order(np.array(segs), self.t)
