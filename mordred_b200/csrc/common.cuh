@@ -135,6 +135,16 @@ __device__ __forceinline__ void smem_add_i64(unsigned long long* sum, int v) {
 __device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void allow_dependent() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// A value of a fact column read for a scattered row. The 64-byte hint keeps DRAM from fetching
+// the whole 128-byte line around it, which is what a plain load does, and the value is not kept
+// in L1. Query B over 24 M rows, four columns gathered at 4 % and 1.6 % of the rows: 338 MB
+// from DRAM against 422 MB (367 against 414 us a call at 120 M rows).
+__device__ __forceinline__ int gather_ld(const int* p) {
+  int v;
+  asm volatile("ld.global.nc.L1::no_allocate.L2::64B.b32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
 __device__ __forceinline__ void set_status(unsigned int* status, unsigned int bits) {
   if (status) atomicOr(status, bits);
 }

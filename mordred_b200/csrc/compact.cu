@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(kSelMaxWarps * 32, 1) select_slices_kernel(con
         if (r == 1 && !two) break;
         q[r * 32] = static_cast<int>(phys) + row[r];
         if (BM) q[kSelQueue + r * 32] = w.stage[NF][row[r]];  // its key: looked up on the way out
-        if (K) h[r] = staged_now ? w.stage[ND][row[r]] : __ldg(cols[NF + kFirst] + idx + row[r]);
+        if (K) h[r] = staged_now ? w.stage[ND][row[r]] : gather_ld(cols[NF + kFirst] + idx + row[r]);
       }
       if (base + kSelRound >= cnt) {
         __syncwarp();  // the buffer has been read: the next slice may land on it
@@ -360,8 +360,8 @@ __global__ void __launch_bounds__(kSelMaxWarps * 32, 1) select_slices_kernel(con
           const int* ht = P.pht[p];
           if (p > kFirst) {
             const int* col = cols[NF + p] + idx;
-            h[0] = __ldg(col + row[0]);
-            if (two) h[1] = __ldg(col + row[1]);
+            h[0] = gather_ld(col + row[0]);
+            if (two) h[1] = gather_ld(col + row[1]);
           }
           int out[2] = {0, 0};
           bool in[2] = {false, false};

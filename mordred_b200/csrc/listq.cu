@@ -142,10 +142,10 @@ __global__ void __launch_bounds__(kListThreads, kListCtas) list_kernel(const __g
         for (int i = 0; i < R; ++i) v[i] = (of >> i) & 1u ? __ldg(col + seg[i]) : 0;
 #pragma unroll
         for (int i = 0; i < R; ++i)
-          v[i] = (of >> i) & 1u ? __ldg(P.gpu_cache + (static_cast<long long>(v[i]) << P.seg_shift) + idx[i]) : 0;
+          v[i] = (of >> i) & 1u ? gather_ld(P.gpu_cache + (static_cast<long long>(v[i]) << P.seg_shift) + idx[i]) : 0;
       } else {
 #pragma unroll
-        for (int i = 0; i < R; ++i) v[i] = (of >> i) & 1u ? __ldg(col + idx[i]) : 0;
+        for (int i = 0; i < R; ++i) v[i] = (of >> i) & 1u ? gather_ld(col + idx[i]) : 0;
       }
     };
     // ---- filters ----

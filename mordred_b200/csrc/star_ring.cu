@@ -394,10 +394,10 @@ __global__ void __launch_bounds__(kRingMaxWarps * 32, 1) star_ring_kernel(const 
         if (P.gpu_cache == nullptr) {
 #pragma unroll
           for (int q = kQ0; q < MB_MAX_PROBES; ++q)
-            if (q < ns) gv[q] = __ldg(P.col[P.p_col[P.sp_ord[q]]] + r);
+            if (q < ns) gv[q] = gather_ld(P.col[P.p_col[P.sp_ord[q]]] + r);
           if (early) {
-            a0 = __ldg(P.col[P.a_col[0]] + r);
-            if (two_cols) a1 = __ldg(P.col[P.a_col[1]] + r);
+            a0 = gather_ld(P.col[P.a_col[0]] + r);
+            if (two_cols) a1 = gather_ld(P.col[P.a_col[1]] + r);
           }
         } else {
           const long long vseg = r >> P.seg_shift;
@@ -413,10 +413,10 @@ __global__ void __launch_bounds__(kRingMaxWarps * 32, 1) star_ring_kernel(const 
           }
 #pragma unroll
           for (int q = kQ0; q < MB_MAX_PROBES; ++q)
-            if (q < ns) gv[q] = __ldg(in_seg + (static_cast<long long>(gv[q]) << P.seg_shift));
+            if (q < ns) gv[q] = gather_ld(in_seg + (static_cast<long long>(gv[q]) << P.seg_shift));
           if (early) {
-            a0 = __ldg(in_seg + (static_cast<long long>(a0) << P.seg_shift));
-            if (two_cols) a1 = __ldg(in_seg + (static_cast<long long>(a1) << P.seg_shift));
+            a0 = gather_ld(in_seg + (static_cast<long long>(a0) << P.seg_shift));
+            if (two_cols) a1 = gather_ld(in_seg + (static_cast<long long>(a1) << P.seg_shift));
           }
         }
         unsigned long long word[MB_MAX_PROBES];
@@ -455,13 +455,13 @@ __global__ void __launch_bounds__(kRingMaxWarps * 32, 1) star_ring_kernel(const 
           if (P.count_after < 0) ++A.cnt;
           if (!early) {
             if (P.gpu_cache == nullptr) {
-              a0 = __ldg(P.col[P.a_col[0]] + r);
-              if (two_cols) a1 = __ldg(P.col[P.a_col[1]] + r);
+              a0 = gather_ld(P.col[P.a_col[0]] + r);
+              if (two_cols) a1 = gather_ld(P.col[P.a_col[1]] + r);
             } else {
               a0 = __ldg(P.col[P.a_col[0]] + seg);
               if (two_cols) a1 = __ldg(P.col[P.a_col[1]] + seg);
-              a0 = __ldg(in_seg + (static_cast<long long>(a0) << P.seg_shift));
-              if (two_cols) a1 = __ldg(in_seg + (static_cast<long long>(a1) << P.seg_shift));
+              a0 = gather_ld(in_seg + (static_cast<long long>(a0) << P.seg_shift));
+              if (two_cols) a1 = gather_ld(in_seg + (static_cast<long long>(a1) << P.seg_shift));
             }
           }
           const unsigned u0 = static_cast<unsigned>(a0), u1 = static_cast<unsigned>(a1);
