@@ -9,8 +9,8 @@
 //     warp waits for another and a slice is on its way while one is worked on;
 //   * dense part: 8 rows a lane, filters and bitmaps into a bit mask a lane;
 //   * the survivors are compacted and the first table probe runs over full lanes, two rows a
-//     lane; the rows it keeps — row number and payload — go to the warp's ring in shared
-//     memory;
+//     lane, its loads in flight under the next slice's dense part; the rows it keeps — row
+//     number and payload — go to the warp's ring in shared memory;
 //   * 32 rows of the ring at a time, one a lane, take the rest of the pipeline: the remaining
 //     keys and the aggregate columns are gathered from the fact columns (all at once), the
 //     remaining tables are probed (all at once), and the sums go to a shared-memory group array
@@ -40,21 +40,21 @@ __host__ __device__ constexpr int ring_warp_bytes(int nst) {
   return static_cast<int>(sizeof(RingWarp)) + 2 * nst * kRingRows * 4;
 }
 
-// The word of slot h >= 0 of a table, 0 when absent. Only the load: callers issue all of a
-// round's before they look at one.
-__device__ __forceinline__ unsigned long long ring_word(const int* ht, int layout, int h) {
-  unsigned long long v;
-  if (layout == MB_HT_KEY)
-    v = static_cast<unsigned>(__ldg(ht + h));
-  else
-    v = ldg_u64(ht + 2ll * h);
-  return v;
+// lo, hi = the word of slot h >= 0 of a table if `on` (0 when absent), else left alone. Only the
+// loads, under opposite predicates: nothing waits for them before their first use.
+__device__ __forceinline__ void ring_word(const int* ht, bool key_layout, int h, bool on, unsigned& lo, unsigned& hi) {
+  asm volatile(
+      "{\n\t.reg .pred k, v;\n\t"
+      "setp.eq.u32 k, %4, 1;\n\t"
+      "setp.eq.u32 v, %4, 2;\n\t"
+      "@k ld.global.nc.u32 %0, [%2];\n\t"
+      "@v ld.global.nc.v2.u32 {%0, %1}, [%3];\n\t}"
+      : "+r"(lo), "+r"(hi)
+      : "l"(ht + h), "l"(ht + 2ll * h), "r"(!on ? 0u : key_layout ? 1u : 2u));
 }
 // The payload in a word, as probe_round's.
-__device__ __forceinline__ int ring_payload(int layout, unsigned long long v) {
-  return layout == MB_HT_KEY_VAL   ? static_cast<int>(v >> 32)
-         : layout == MB_HT_VAL_OFF ? static_cast<int>(static_cast<unsigned>(v))
-                                   : 0;
+__device__ __forceinline__ int ring_payload(int layout, unsigned lo, unsigned hi) {
+  return static_cast<int>(layout == MB_HT_KEY_VAL ? hi : layout == MB_HT_VAL_OFF ? lo : 0u);
 }
 
 // Adds a row to the groups: `hh` its group index, val its value; keys written for the first
@@ -229,6 +229,9 @@ __global__ void __launch_bounds__(kRingMaxWarps * 32, 1) star_ring_kernel(const 
   __syncthreads();
 
   int held = 0;  // rows in the ring
+  // the round of the first table probe in flight: its table words (0: no survivor) and rows
+  unsigned plo[2] = {0, 0}, phi[2] = {0, 0};
+  int prow[2] = {0, 0};
   for (uint32_t it = 0;; ++it, s += nwarps) {
     const bool drain = s >= s_end || failed;  // one more step after the last slice empties the ring
     const int buf = it & 1;
@@ -319,60 +322,17 @@ __global__ void __launch_bounds__(kRingMaxWarps * 32, 1) star_ring_kernel(const 
     }
     int base = 0;
     do {
-      // ---- the first table probe: entries base + r * 32 + lane (an absent one reads row 0) ----
-      int row[2] = {0, 0}, pay[2] = {0, 0};
-      bool ok[2] = {false, false};
-      if (!drain) {
-        int key[2] = {0, 0};
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          const int e = base + r * 32 + lane;
-          ok[r] = e < cnt;
-          row[r] = ok[r] ? w.off[e] : 0;
-          if (K) key[r] = st[P.r_kcol * kRingRows + row[r]];
-        }
-        if (base + kRingRound >= cnt) {
-          __syncwarp();  // the buffer has been read: another slice may land on it
-          if (s + 2 * nwarps < s_end && !failed) start(s + 2 * nwarps, buf);
-        }
-        if (K) {
-          const int p = P.sp_ord[0];
-          const int* ht = P.p_ht[p];
-          const int layout = P.p_layout[p];
-          int h[2];
-#pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            h[r] = pht_slot(key[r], P.p_slots[p], P.p_kmin[p]);
-            if (h[r] < 0) {
-              if (ok[r]) A.bad_probe = true;
-              ok[r] = false;
-              h[r] = 0;
-            }
-            if (!ok[r]) h[r] = 0;
-          }
-          unsigned long long word[2];
-          if (layout == MB_HT_KEY) {
-            word[0] = ring_word(ht, MB_HT_KEY, h[0]);
-            word[1] = ring_word(ht, MB_HT_KEY, h[1]);
-          } else {
-            word[0] = ring_word(ht, MB_HT_KEY_VAL, h[0]);
-            word[1] = ring_word(ht, MB_HT_KEY_VAL, h[1]);
-          }
-#pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            ok[r] = ok[r] && word[r] != 0ull;
-            pay[r] = ring_payload(layout, word[r]);
-          }
-        }
-      }
-      const uint32_t b0 = __ballot_sync(kFull, ok[0]), b1 = __ballot_sync(kFull, ok[1]);
+      // ---- the round probed last: its survivors to the ring ----
+      const bool ok0 = (plo[0] | phi[0]) != 0u, ok1 = (plo[1] | phi[1]) != 0u;
+      const uint32_t b0 = __ballot_sync(kFull, ok0), b1 = __ballot_sync(kFull, ok1);
       const int add = __popc(b0) + __popc(b1);
       bool pushed = add == 0;
       while (true) {
         if (!pushed && held + add <= kRingCap) {
-          const int r0 = s * kRingRows;
-          if (ok[0]) w.ring[held + __popc(b0 & below)] = make_int2(pay[0], r0 + row[0]);
-          if (ok[1]) w.ring[held + __popc(b0) + __popc(b1 & below)] = make_int2(pay[1], r0 + row[1]);
+          const int layout = K ? P.p_layout[P.sp_ord[0]] : MB_HT_KEY;
+          if (ok0) w.ring[held + __popc(b0 & below)] = make_int2(ring_payload(layout, plo[0], phi[0]), prow[0]);
+          if (ok1)
+            w.ring[held + __popc(b0) + __popc(b1 & below)] = make_int2(ring_payload(layout, plo[1], phi[1]), prow[1]);
           held += add;
           pushed = true;
           __syncwarp();
@@ -419,37 +379,25 @@ __global__ void __launch_bounds__(kRingMaxWarps * 32, 1) star_ring_kernel(const 
             if (two_cols) a1 = gather_ld(in_seg + (static_cast<long long>(a1) << P.seg_shift));
           }
         }
-        unsigned long long word[MB_MAX_PROBES];
+        unsigned lo[MB_MAX_PROBES], hi[MB_MAX_PROBES];
         bool below_min[MB_MAX_PROBES];
 #pragma unroll
         for (int q = kQ0; q < MB_MAX_PROBES; ++q) {
-          word[q] = 1ull;
+          lo[q] = hi[q] = 0;
           below_min[q] = false;
           if (q < ns) {
             const int p = P.sp_ord[q];
-            int h = pht_slot(gv[q], P.p_slots[p], P.p_kmin[p]);
+            const int h = pht_slot(gv[q], P.p_slots[p], P.p_kmin[p]);
             below_min[q] = h < 0;
-            h = max(h, 0);
-            // two loads under opposite predicates, so that the probes share one basic block
-            const int* ht = P.p_ht[p];
-            const bool key = P.p_layout[p] == MB_HT_KEY;
-            unsigned lo = 0, hi = 0;
-            asm volatile(
-                "{\n\t.reg .pred k;\n\t"
-                "setp.ne.u32 k, %4, 0;\n\t"
-                "@k ld.global.nc.u32 %0, [%2];\n\t"
-                "@!k ld.global.nc.v2.u32 {%0, %1}, [%3];\n\t}"
-                : "+r"(lo), "+r"(hi)
-                : "l"(ht + h), "l"(ht + 2ll * h), "r"(key ? 1u : 0u));
-            word[q] = (static_cast<unsigned long long>(hi) << 32) | lo;
+            ring_word(P.p_ht[p], P.p_layout[p] == MB_HT_KEY, h, h >= 0, lo[q], hi[q]);
           }
         }
 #pragma unroll
         for (int q = kQ0; q < MB_MAX_PROBES; ++q) {
           if (q >= ns) continue;
           if (live && below_min[q]) A.bad_probe = true;
-          live = live && !below_min[q] && word[q] != 0ull;
-          gv[q] = ring_payload(P.p_layout[P.sp_ord[q]], word[q]);
+          live = live && (lo[q] | hi[q]) != 0u;
+          gv[q] = ring_payload(P.p_layout[P.sp_ord[q]], lo[q], hi[q]);
         }
         if (live) {
           if (P.count_after < 0) ++A.cnt;
@@ -479,6 +427,37 @@ __global__ void __launch_bounds__(kRingMaxWarps * 32, 1) star_ring_kernel(const 
           }
         }
         __syncwarp();  // the rows are read before others take their places
+      }
+      // ---- the next round of the first table probe: entries base + r * 32 + lane of the
+      // survivors (an absent one reads row 0). Its table words are looked at when the next
+      // round begins, after the next slice's dense part where this was the slice's last ----
+      plo[0] = phi[0] = plo[1] = phi[1] = 0;
+      if (!drain) {
+        int row[2], key[2];
+        bool ok[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int e = base + r * 32 + lane;
+          ok[r] = e < cnt;
+          row[r] = ok[r] ? w.off[e] : 0;
+          key[r] = K ? st[P.r_kcol * kRingRows + row[r]] : 0;
+        }
+        if (base + kRingRound >= cnt) {
+          __syncwarp();  // the buffer has been read: another slice may land on it
+          if (s + 2 * nwarps < s_end && !failed) start(s + 2 * nwarps, buf);
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          prow[r] = s * kRingRows + row[r];
+          if (K) {
+            const int p = P.sp_ord[0];
+            const int h = pht_slot(key[r], P.p_slots[p], P.p_kmin[p]);
+            if (h < 0 && ok[r]) A.bad_probe = true;
+            ring_word(P.p_ht[p], P.p_layout[p] == MB_HT_KEY, h, ok[r] && h >= 0, plo[r], phi[r]);
+          } else {
+            plo[r] = ok[r] ? 1u : 0u;
+          }
+        }
       }
       base += kRingRound;
     } while (base < cnt);
