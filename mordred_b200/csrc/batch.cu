@@ -43,6 +43,11 @@ constexpr int kSmemTableMaxEntries = 512;  // predicate tables up to this many v
 constexpr int kCombineMaxEntries = 320;    // entries of a table that combines several small attributes
 constexpr int kMaxComponents = 4;          // attributes a table combines
 constexpr int kMaxClasses = 4;
+// Shared memory the default group placement fills at most: what is left of the SM's 256 KB is L1,
+// and the dimension lookups of every row miss it — with 28 KB of L1 few can be in flight. 256
+// queries over 20 M rows, group arrays up to 32 KB (60 KB of L1) 1.84 ms, 64 KB and more 2.20;
+// date-sorted 1.73 and 2.05.
+constexpr int kSmemBesideL1 = 195 * 1024;
 constexpr int kMatchListCap = 512;         // pairs of one class a consumer warp collects before aggregating
 constexpr int kColPad = 4;                 // words between staged columns: the same row of two columns
                                            // falls in different banks (and stays 16-byte aligned)
@@ -1381,6 +1386,7 @@ extern "C" int mb_batch_run(const mb_batch_args* a, mb_stream_t stream) {
   P.smem_groups_off = off;
   int groups_bytes = 0;
   const int group_cap = a->smem_group_bytes < 0 ? 131072 : a->smem_group_bytes;
+  const int group_budget = a->smem_group_bytes < 0 && budget > kSmemBesideL1 ? kSmemBesideL1 : budget;
   // shared memory kept for the touch bitmaps of the small-array queries that end up with
   // L2 sums (below): a few bytes each, and without one such a query writes its keys on
   // every match
@@ -1407,7 +1413,7 @@ extern "C" int mb_batch_run(const mb_batch_args* a, mb_stream_t stream) {
       const AQ& A = P.q[qi].a;
       if (P.q[qi].res_layout == MB_RES_SCALAR || A.soff >= 0 || A.total != total) continue;
       if (groups_bytes + fam_bytes(members + 1) > group_cap ||
-          total_smem(off + groups_bytes + fam_bytes(members + 1) + touch_reserve, stages) > budget)
+          total_smem(off + groups_bytes + fam_bytes(members + 1) + touch_reserve, stages) > group_budget)
         break;
       ++members;
     }
