@@ -162,6 +162,7 @@ class StarWorkspace:
     def __post_init__(self):
         z = lambda n: torch.zeros(n, dtype=torch.int32, device=self.device)
         s = self.sizes
+        scalars = torch.zeros(2, dtype=torch.int64, device=self.device)
         self.t = {
             "ht_s": z(s.s_len),                # MB_HT_KEY (supplier existence)
             "ht_c": z(2 * s.c_len),            # MB_HT_KEY_VAL (custkey -> nation)
@@ -170,8 +171,9 @@ class StarWorkspace:
             "ht_d": z(2 * self.date_slots),    # MB_HT_KEY_VAL (datekey -> year)
             "res_a": z(4 * QA_GROUPS),
             "res_b": z(4 * QB_GROUPS),
-            "rev": torch.zeros(1, dtype=torch.int64, device=self.device),
-            "cnt": torch.zeros(1, dtype=torch.int32, device=self.device),
+            "scalars": scalars,                # rev and cnt: one buffer, cleared in one launch
+            "rev": scalars[:1],
+            "cnt": scalars[1:].view(torch.int32)[:1],
         }
 
     def __getitem__(self, k):
@@ -180,11 +182,13 @@ class StarWorkspace:
 
 def q11(t: dict, n: int, ws: StarWorkspace | None = None, stream=None, zero=True) -> torch.Tensor:
     """Filter-aggregate (src/ssb/q11.cu). Returns the device uint64 revenue (int64 tensor)."""
-    rev = ws["rev"] if ws is not None else torch.zeros(1, dtype=torch.int64, device=t["lo_orderdate"].device)
-    cnt = ws["cnt"] if ws is not None else torch.zeros(1, dtype=torch.int32, device=rev.device)
-    if zero:
-        rev.zero_()
-        cnt.zero_()
+    if ws is not None:
+        rev, cnt = ws["rev"], ws["cnt"]
+        if zero:
+            ws["scalars"].zero_()
+    else:
+        rev = torch.zeros(1, dtype=torch.int64, device=t["lo_orderdate"].device)
+        cnt = torch.zeros(1, dtype=torch.int32, device=rev.device)
     L.call("mb_q11_query", _p(t["lo_orderdate"]), _p(t["lo_discount"]), _p(t["lo_quantity"]),
            _p(t["lo_extendedprice"]), n, _p(rev), _p(cnt), _stream(stream))
     return rev
