@@ -20,6 +20,12 @@
 //     16-byte record of the query — its scalar or shared-memory group array (flushed once
 //     per CTA) or its group array in L2. Queries beyond the four largest classes are
 //     aggregated from a 32-byte descriptor of their own.
+// What bounds it: instruction issue, with the shared-memory pipe behind it (mask reads, match
+// lists, the sums' atomics): 64 and 60 % issue-active at 256 and 24 queries. With a descriptor
+// read for every match and a mask table for every attribute, the form before, the warps issued
+// 80 instructions a row for 256 queries and 23 for 24; now 69 and 15. 256 queries over 60 M rows
+// 6,940 -> 5,230 us a call, over 20 M date-sorted rows 2,500 -> 1,650; 24 queries over a
+// date-sorted chunk of 75 M rows 3,130 -> 1,950.
 // A query's result equals its lone run through mb_star_query with filtered hash tables:
 // with unique dimension keys, "the key is in the filtered table" is "the row's
 // attributes pass the filter", and the payload is the attribute itself; sums are
@@ -788,7 +794,7 @@ __global__ void __launch_bounds__((NCW + 1) * 32, 1) batch_kernel(const __grid_c
 // there (no value outside an attribute's hull passes a predicate on it). A warp takes 32
 // entries of one table and one word: lane l knows the values of the l-th entry and the ranges
 // of the l-th query, and entry by entry the values are broadcast and the verdicts balloted
-// (256 queries: 8 us; each thread walking all queries' descriptors: 70 us).
+// (256 queries: 13.8 us, 24 queries: 8.4; each thread walking all queries' descriptors: 70 and 8.5).
 __global__ void batch_mask_kernel(const __grid_constant__ BatchPlan P, int tasks) {
   const int lane = threadIdx.x & 31;
   allow_dependent();
@@ -1301,8 +1307,9 @@ extern "C" int mb_batch_run(const mb_batch_args* a, mb_stream_t stream) {
   // Defaults: up to 64 queries a row has few matches and the work per row decides, so a lane
   // takes two rows at a time (24 queries over 75 M rows: 768x2 1.76 ms, 960x1 2.22, 768x1
   // 2.52); above, the match lists are full anyway and one more warp a scheduler hides more
-  // (120 queries over 20 M rows: 960x1 1.10 ms, 768x1 1.20, 768x2 1.33; 256 queries: 2.21,
-  // 2.30, 2.21). A call that sets one of the two gets 768 threads or one row for the other.
+  // (120 queries over 20 M rows: 960x1 1.10 ms, 768x1 1.20, 768x2 1.33; 256 queries, with
+  // group arrays filling the shared memory: 2.21, 2.30, 2.21). A call that sets one of the
+  // two gets 768 threads or one row for the other.
   const bool by_size = a->threads == 0 && a->items_per_thread == 0;
   const int threads = a->threads ? a->threads : by_size && P.nwords > 2 ? 960 : 768;
   const int items = a->items_per_thread ? a->items_per_thread : by_size && P.nwords <= 2 ? 2 : 1;
@@ -1397,7 +1404,22 @@ extern "C" int mb_batch_run(const mb_batch_args* a, mb_stream_t stream) {
       touch_reserve += (4 * ((A.total + 31) / 32) + 15) / 16 * 16;
   }
   // queries with the same group count form a family (group-major interleaved sums); as
-  // many members as fit, smallest group counts first
+  // many members as fit, smallest group counts first, and of a family the queries that most
+  // rows can match: its share of the values its predicates' attributes have in this batch.
+  // Sums by L2 atomics of a query that matches often meet on a few lines. 256 queries over 40 M
+  // rows, three draws: the first queries that fit 5.13, 4.00 and 4.88 ms, the widest ones
+  // 3.53, 3.49 and 4.24.
+  float share[MB_BATCH_MAX_QUERIES];
+  for (int qi = 0; qi < P.nq; ++qi) {
+    const BQ& Q = P.q[qi];
+    share[qi] = 1.0f;
+    for (int k = 0; k < Q.np; ++k)
+      for (int f = 0; f < P.nfields; ++f) {
+        if (P.at[f].code != Q.pf[k]) continue;
+        const long long width = static_cast<long long>(Q.phi[k]) - Q.plo[k] + 1;
+        share[qi] *= width > 0 ? static_cast<float>(width) / static_cast<float>(P.at[f].n > 0 ? P.at[f].n : 1) : 0.0f;
+      }
+  }
   for (;;) {
     int total = 0;
     for (int qi = 0; qi < P.nq; ++qi) {
@@ -1417,11 +1439,21 @@ extern "C" int mb_batch_run(const mb_batch_args* a, mb_stream_t stream) {
         break;
       ++members;
     }
+    short by_share[MB_BATCH_MAX_QUERIES];
+    bool chosen[MB_BATCH_MAX_QUERIES] = {};
+    int candidates = 0;
+    for (int qi = 0; qi < P.nq; ++qi) {
+      const AQ& A = P.q[qi].a;
+      if (P.q[qi].res_layout != MB_RES_SCALAR && A.soff < 0 && A.total == total)
+        by_share[candidates++] = static_cast<short>(qi);
+    }
+    std::stable_sort(by_share, by_share + candidates, [&](short x, short y) { return share[x] > share[y]; });
+    for (int i = 0; i < members; ++i) chosen[by_share[i]] = true;
     int j = 0;
     for (int qi = 0; qi < P.nq; ++qi) {
       AQ& A = P.q[qi].a;
       if (P.q[qi].res_layout == MB_RES_SCALAR || A.soff >= 0 || A.total != total) continue;
-      if (j < members) {
+      if (chosen[qi]) {
         A.soff = off + groups_bytes + 8 * j;
         A.flags = (A.flags & 0xff) | ((members | 1) << 8) | (j << 17);
         ++j;
