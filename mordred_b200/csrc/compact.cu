@@ -63,8 +63,8 @@ __device__ __forceinline__ bool sel_pass(int x, int mode, int c1, int c2) {
 // that pass everything wait in the warp's queue and leave 64 at a time: one atomicAdd on the
 // list cursor and full 128-byte stores per 64 rows; a probe the bitmap decided reads its
 // output there.
-// 24,000,000 rows with a date filter and two probes: 90 us, bound by instruction issue and the
-// L2 trips of a round (1.9 warp instructions a row, 43 % issue; DRAM 293 MB, 3.2 TB/s). One
+// 24,000,000 rows with a date filter and two probes: 85 us, bound by instruction issue and the
+// L2 trips of a round (1.9 warp instructions a row, 51 % issue; DRAM 293 MB, 3.4 TB/s). One
 // row a lane with every load behind a branch, and an atomic per 32 rows: 8.8 warp
 // instructions a row, 448 us.
 constexpr int kSelMaxWarps = 32;          // one CTA an SM: the bitmap is derived once an SM

@@ -26,8 +26,9 @@
 // chain's. Group accumulation is the star kernel's: 64-bit sums in a shared-memory group
 // array flushed once per CTA, or L2 atomics for large group arrays; scalars reduced per CTA.
 // 2,000,003 entries over 24,000,000 rows (segment cache, two table probes, one passed-through
-// value): one entry at a time behind branches 127 us; in rounds 76 us. Its entries lie 12 rows
-// apart, so the four gathered columns come in nearly whole (343 MB, 52 us at the copy rate).
+// value): one entry at a time behind branches 127 us; in rounds 76 us; with the 64-byte fetches
+// of gather_ld about 69 (74 a call, from 140). Its entries lie 12 rows apart, so the four
+// gathered columns come in nearly whole (340 MB, 52 us at the copy rate).
 #include <cstring>
 #include <type_traits>
 
@@ -36,7 +37,7 @@
 namespace mb {
 
 // Two entries a thread at three CTAs an SM is what the registers carry without spilling
-// (2,000,003 entries: 81 us a call; 4 entries at 3 CTAs 113 us and 2 at 4 CTAs 93 us, both
+// (2,000,003 entries, plain gathers: 81 us a call; 4 entries at 3 CTAs 113 us and 2 at 4 CTAs 93 us, both
 // spilling; 4 at 2 CTAs 80 us, but 133 against 123 us for 4.8 M entries).
 constexpr int kListItems = 2;
 constexpr int kListThreads = 256;
