@@ -995,57 +995,9 @@ static int plan_batch(const mb_batch_args* a, BatchPlan& P, bool sizing) {
     d.res = q.res;
     req[qi] = static_cast<unsigned>(q.dims_required);
   }
-  // Classes: queries that add the same expression to the same group index, most members
-  // first. The queries are renumbered class by class, so that a class's bits share few words.
-  int cls_of[MB_BATCH_MAX_QUERIES], first_of[MB_BATCH_MAX_QUERIES], members[MB_BATCH_MAX_QUERIES], nfound = 0;
-  for (int qi = 0; qi < P.nq && !sizing; ++qi) {
-    auto same = [&](int o) {
-      const AQ &A = P.q[qi].a, &C = P.q[o].a;
-      return af[qi][0] == af[o][0] && af[qi][1] == af[o][1] && kf[qi][0] == kf[o][0] && kf[qi][1] == kf[o][1] &&
-             A.kmul0 == C.kmul0 && A.kmul1 == C.kmul1 && A.bias == C.bias && A.total == C.total && A.flags == C.flags;
-    };
-    int c = 0;
-    while (c < nfound && !same(first_of[c])) ++c;
-    if (c == nfound) {
-      first_of[nfound] = qi;
-      members[nfound++] = 0;
-    }
-    ++members[c];
-    cls_of[qi] = c;
-  }
-  if (!sizing) {
-    int rank[MB_BATCH_MAX_QUERIES], order[MB_BATCH_MAX_QUERIES], next[kMaxClasses + 1] = {0};
-    for (int c = 0; c < nfound; ++c) rank[c] = kMaxClasses;
-    for (int i = 0; i < kMaxClasses && i < nfound; ++i) {
-      int best = -1;
-      for (int c = 0; c < nfound; ++c)
-        if (rank[c] == kMaxClasses && (best < 0 || members[c] > members[best])) best = c;
-      rank[best] = i;
-    }
-    for (int qi = 0; qi < P.nq; ++qi) {
-      cls_of[qi] = rank[cls_of[qi]];
-      for (int c = cls_of[qi] + 1; c <= kMaxClasses; ++c) ++next[c];
-    }
-    for (int qi = 0; qi < P.nq; ++qi) order[next[cls_of[qi]]++] = qi;
-    P.ncls = nfound < kMaxClasses ? nfound : kMaxClasses;
-    P.others = nfound > kMaxClasses ? 1 : 0;
-    std::vector<BQ> q0(P.q, P.q + P.nq);
-    std::vector<int> from(6 * P.nq);
-    for (int qi = 0; qi < P.nq; ++qi) {
-      int* f = &from[6 * qi];
-      f[0] = af[qi][0], f[1] = af[qi][1], f[2] = kf[qi][0], f[3] = kf[qi][1];
-      f[4] = static_cast<int>(req[qi]), f[5] = cls_of[qi];
-    }
-    for (int qi = 0; qi < P.nq; ++qi) {
-      const int* f = &from[6 * order[qi]];
-      P.q[qi] = q0[order[qi]];
-      af[qi][0] = f[0], af[qi][1] = f[1], kf[qi][0] = f[2], kf[qi][1] = f[3];
-      req[qi] = static_cast<unsigned>(f[4]), cls_of[qi] = f[5];
-      P.cls_mask[cls_of[qi]][qi / 32] |= 1u << (qi % 32);
-      P.all[qi / 32] |= 1u << (qi % 32);
-    }
-  }
-  // constrained attributes and the hull of the ranges on each
+  // Constrained attributes, the hull of the ranges on each, and interval coding, which goes to
+  // wide attributes in the order the caller's queries first name them: before the queries are
+  // renumbered, so that sizing the workspace and running the batch plan the same tables.
   Attr attr[kMaxPredFields] = {};
   int hmin[kMaxPredFields], hmax[kMaxPredFields];
   bool has[kMaxPredFields] = {false};
@@ -1104,6 +1056,56 @@ static int plan_batch(const mb_batch_args* a, BatchPlan& P, bool sizing) {
         while ((static_cast<long long>(kMaxBuckets) << shift) < n) ++shift;
         A.bkt_shift = shift;
       }
+    }
+  }
+  // Classes: queries that add the same expression to the same group index, most members
+  // first. The queries are renumbered class by class, so that a class's bits share few words.
+  int cls_of[MB_BATCH_MAX_QUERIES], first_of[MB_BATCH_MAX_QUERIES], members[MB_BATCH_MAX_QUERIES], nfound = 0;
+  for (int qi = 0; qi < P.nq && !sizing; ++qi) {
+    auto same = [&](int o) {
+      const AQ &A = P.q[qi].a, &C = P.q[o].a;
+      return af[qi][0] == af[o][0] && af[qi][1] == af[o][1] && kf[qi][0] == kf[o][0] && kf[qi][1] == kf[o][1] &&
+             A.kmul0 == C.kmul0 && A.kmul1 == C.kmul1 && A.bias == C.bias && A.total == C.total && A.flags == C.flags;
+    };
+    int c = 0;
+    while (c < nfound && !same(first_of[c])) ++c;
+    if (c == nfound) {
+      first_of[nfound] = qi;
+      members[nfound++] = 0;
+    }
+    ++members[c];
+    cls_of[qi] = c;
+  }
+  if (!sizing) {
+    int rank[MB_BATCH_MAX_QUERIES], order[MB_BATCH_MAX_QUERIES], next[kMaxClasses + 1] = {0};
+    for (int c = 0; c < nfound; ++c) rank[c] = kMaxClasses;
+    for (int i = 0; i < kMaxClasses && i < nfound; ++i) {
+      int best = -1;
+      for (int c = 0; c < nfound; ++c)
+        if (rank[c] == kMaxClasses && (best < 0 || members[c] > members[best])) best = c;
+      rank[best] = i;
+    }
+    for (int qi = 0; qi < P.nq; ++qi) {
+      cls_of[qi] = rank[cls_of[qi]];
+      for (int c = cls_of[qi] + 1; c <= kMaxClasses; ++c) ++next[c];
+    }
+    for (int qi = 0; qi < P.nq; ++qi) order[next[cls_of[qi]]++] = qi;
+    P.ncls = nfound < kMaxClasses ? nfound : kMaxClasses;
+    P.others = nfound > kMaxClasses ? 1 : 0;
+    std::vector<BQ> q0(P.q, P.q + P.nq);
+    std::vector<int> from(6 * P.nq);
+    for (int qi = 0; qi < P.nq; ++qi) {
+      int* f = &from[6 * qi];
+      f[0] = af[qi][0], f[1] = af[qi][1], f[2] = kf[qi][0], f[3] = kf[qi][1];
+      f[4] = static_cast<int>(req[qi]), f[5] = cls_of[qi];
+    }
+    for (int qi = 0; qi < P.nq; ++qi) {
+      const int* f = &from[6 * order[qi]];
+      P.q[qi] = q0[order[qi]];
+      af[qi][0] = f[0], af[qi][1] = f[1], kf[qi][0] = f[2], kf[qi][1] = f[3];
+      req[qi] = static_cast<unsigned>(f[4]), cls_of[qi] = f[5];
+      P.cls_mask[cls_of[qi]][qi / 32] |= 1u << (qi % 32);
+      P.all[qi / 32] |= 1u << (qi % 32);
     }
   }
   if (!sizing) {

@@ -1,0 +1,37 @@
+"""Batches at the limits of the planner — end points and shared memory run out — sized by
+mb_batch_workspace_bytes and checked against a plain numpy evaluation of every query."""
+import numpy as np
+import pytest
+
+import test_batch_masks as M
+from mordred_b200 import _lib as L
+from mordred_b200 import batch as B
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(n, queries, seed, ranges=(), **launch):
+    """`ranges`: fact columns drawn anew, (name, values)."""
+    t, words = M._data(n, seed, 0.9)
+    rng = np.random.default_rng(seed + 1)
+    for name, values in ranges:
+        t[name] = rng.integers(0, values, n).astype(np.int64)
+    L.device_status(0)
+    got = M._run(t, words, queries, n, **launch)
+    for i, (q, g) in enumerate(zip(queries, got)):
+        assert M._same(q, g, M._expected(q, t, words)), (i, q)
+    assert L.device_status(0) == 0
+
+
+@pytest.mark.parametrize("count", [200, 256])
+def test_more_end_points_than_fit_named_in_different_orders(count):
+    """Two wide attributes with more than 768 end points together. The first query is of a class
+    of its own and names the quantity; the others, the largest class, name the part first."""
+    part, quantity = B.F(L.MB_COL_DIM_P, 5, 10), B.FACT["lo_quantity"]
+    grouped = dict(layout=L.MB_RES_CRYSTAL4, keys=[(B.F(L.MB_COL_DIM_D, 0, 4), 0, 1)], op=L.MB_AGG_SUM,
+                   agg=[B.FACT["lo_revenue"]], total=16, dims=12)
+    queries = [dict(layout=L.MB_RES_SCALAR, keys=[], op=L.MB_AGG_SUB, agg=[B.FACT["lo_revenue"], B.FACT["lo_supplycost"]],
+                    total=1, dims=0, preds=[(quantity, 0, 3_999)])]
+    for i in range(1, count):
+        queries.append(dict(grouped, preds=[(part, i, 1_023 - i), (quantity, 2 * i, 3_999 - 3 * i)]))
+    _check(7_001, queries, count, ranges=[("lo_quantity", 4_000)])
