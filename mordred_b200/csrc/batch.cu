@@ -1463,7 +1463,7 @@ extern "C" int mb_batch_run(const mb_batch_args* a, mb_stream_t stream) {
         A.flags |= 1 << 30;  // no room: sums by L2 atomics (marked so the search moves on)
       }
     }
-    groups_bytes += fam_bytes(members);
+    if (members > 0) groups_bytes += fam_bytes(members);  // a family without room takes none
   }
   for (int qi = 0; qi < P.nq; ++qi) P.q[qi].a.flags &= ~(1 << 30);
   // queries left with L2 sums that write keys, and few groups (a few hot result lines),

@@ -35,3 +35,15 @@ def test_more_end_points_than_fit_named_in_different_orders(count):
     for i in range(1, count):
         queries.append(dict(grouped, preds=[(part, i, 1_023 - i), (quantity, 2 * i, 3_999 - 3 * i)]))
     _check(7_001, queries, count, ranges=[("lo_quantity", 4_000)])
+
+
+@pytest.mark.parametrize("smem", [-1, 0, 131_072])
+@pytest.mark.parametrize("count", [16, 40])
+def test_more_group_counts_than_shared_memory_holds(count, smem):
+    """Every query has a group count of its own, near 1,000: most get no shared-memory sums."""
+    year, brand = B.F(L.MB_COL_DIM_D, 0, 4), B.F(L.MB_COL_DIM_P, 4, 6)
+    queries = [dict(layout=[L.MB_RES_DENSE, L.MB_RES_CRYSTAL4][i % 2], keys=[(year, 0, 1), (brand, 0, 16)],
+                    op=L.MB_AGG_SUB, agg=[B.FACT["lo_revenue"], B.FACT["lo_supplycost"]], total=1_024 - i, dims=15,
+                    preds=[(B.FACT["lo_quantity"], i % 7, 49), (B.FACT["lo_discount"], -3, 13 - i % 5)])
+               for i in range(count)]
+    _check(5_003, queries, count, smem_group_bytes=smem)
