@@ -1313,35 +1313,15 @@ extern "C" int mb_batch_run(const mb_batch_args* a, mb_stream_t stream) {
   // group arrays filling the shared memory: 2.21, 2.30, 2.21). A call that sets one of the
   // two gets 768 threads or one row for the other.
   const bool by_size = a->threads == 0 && a->items_per_thread == 0;
-  const int threads = a->threads ? a->threads : by_size && P.nwords > 2 ? 960 : 768;
-  const int items = a->items_per_thread ? a->items_per_thread : by_size && P.nwords <= 2 ? 2 : 1;
-  const int nwm = P.nwords;
-  const BatchVariant* var = nullptr;
-  for (const BatchVariant& v : kBatchVariants)
-    if (v.warps * 32 == threads && v.items == items && v.nwm == nwm) var = &v;
-  if (var == nullptr) return MB_ERR_ARG;
-  const int tile = threads * items;
-  P.nfull = P.n / tile;
-  // stage word offsets
-  auto field = [&](int code) {
-    const int width = code & 63;
-    return Field{(code >> 11) * (tile + kColPad), (code >> 6) & 31, width >= 32 ? 0xffffffffu : (1u << width) - 1u};
+  int threads = a->threads ? a->threads : by_size && P.nwords > 2 ? 960 : 768;
+  int items = a->items_per_thread ? a->items_per_thread : by_size && P.nwords <= 2 ? 2 : 1;
+  auto variant = [&]() -> const BatchVariant* {
+    for (const BatchVariant& v : kBatchVariants)
+      if (v.warps * 32 == threads && v.items == items && v.nwm == P.nwords) return &v;
+    return nullptr;
   };
-  for (int f = 0; f < P.nfields; ++f) P.at[f].f = field(P.at[f].scode);
-  for (int j = 0; j < P.ndims; ++j) {
-    P.dim[j].key_word *= tile + kColPad;
-    P.dim[j].word *= tile + kColPad;
-  }
-  for (int c = 0; c < P.ncls; ++c) {
-    int qi = 0;  // its first query
-    while (!((P.cls_mask[c][qi / 32] >> (qi % 32)) & 1u)) ++qi;
-    const AQ& A = P.q[qi].a;
-    P.cls[c] = {field(A.a0), field(A.a1), field(A.k0), field(A.k1), A.kmul0, A.kmul1, A.bias,
-                A.total, A.flags & 3, (A.flags >> 5) & 1, ((A.flags >> 3) & 3) > 1 ? 1 : 0};
-  }
-  P.stage_words = (P.ncols + ((P.ndims && P.dim[P.ndims - 1].d == 3) ? 1 : 0)) * (tile + kColPad);
   int stages = a->stages ? a->stages : 2;
-  if (stages < 2 || stages > kBatchStages) return MB_ERR_ARG;
+  if (variant() == nullptr || stages < 2 || stages > kBatchStages) return MB_ERR_ARG;
 
   // shared memory: barriers | scalars | aggregation descriptors | match records | result
   // pointers | sum addresses | presence masks | predicate tables | match lists | small
@@ -1365,26 +1345,67 @@ extern "C" int mb_batch_run(const mb_batch_args* a, mb_stream_t stream) {
   P.smem_pres_off = off;
   off += 16 * kMaskWordsMax * 4;
   const int budget = ds->max_smem_optin - 2048;
-  auto total_smem = [&](int base, int st) { return (base + 127) / 128 * 128 + st * P.stage_words * 4; };
-  for (int f = 0; f < P.nfields; ++f) {
-    Attr& A = P.at[f];
-    if (A.nint > 0) {
-      A.bps_off = off;
-      off += (A.nint * 4 + 15) / 16 * 16;
-      A.bkt_off = off;
-      off += ((((A.n - 1) >> A.bkt_shift) + 1) * 2 + 15) / 16 * 16;
+  const int stage_cols = P.ncols + (P.ndims && P.dim[P.ndims - 1].d == 3 ? 1 : 0);
+  const int tables_off = off;
+  bool in_smem[kMaxPredFields];
+  for (int f = 0; f < P.nfields; ++f)  // single attributes with too many values and end points stay in the workspace
+    in_smem[f] = P.at[f].last && (P.at[f].nint > 0 || P.at[f].ent <= kSmemTableMaxEntries + 1);
+  auto place_tables = [&] {
+    off = tables_off;
+    for (int f = 0; f < P.nfields; ++f) {
+      Attr& A = P.at[f];
+      if (A.nint > 0) {
+        A.bps_off = off;
+        off += (A.nint * 4 + 15) / 16 * 16;
+        A.bkt_off = off;
+        off += ((((A.n - 1) >> A.bkt_shift) + 1) * 2 + 15) / 16 * 16;
+      }
+      A.smem_off = in_smem[f] ? off : -1;
+      if (in_smem[f]) off += (A.ent * P.nwords * 4 + 15) / 16 * 16;
     }
-    if (!A.last) continue;
-    // single attributes with too many values and end points stay in the workspace
-    A.smem_off = -1;
-    if (A.nint == 0 && A.ent > kSmemTableMaxEntries + 1) continue;
-    A.smem_off = off;
-    off += (A.ent * P.nwords * 4 + 15) / 16 * 16;
+  };
+  place_tables();
+  auto fits = [&](int st) {
+    const int lists = threads / 32 * kMatchListCap * 2;
+    return (off + lists + 127) / 128 * 128 + st * stage_cols * (threads * items + kColPad) * 4 <= budget;
+  };
+  // What does not fit takes less, at the cost of speed: a default launch the smaller shape, then
+  // the largest tables stay in the workspace too, until the launch fits.
+  if (by_size && !fits(2)) threads = 768, items = 1;
+  while (!fits(2)) {
+    int most = -1;
+    for (int f = 0; f < P.nfields; ++f)
+      if (in_smem[f] && (most < 0 || P.at[f].ent > P.at[most].ent)) most = f;
+    if (most < 0) return MB_ERR_SIZE;
+    in_smem[most] = false;
+    place_tables();
   }
+  while (!fits(stages)) --stages;
   P.smem_list_off = off;
   off += (threads / 32) * kMatchListCap * 2;
-  while (total_smem(off, stages) > budget && stages > 2) --stages;
-  if (total_smem(off, stages) > budget) return MB_ERR_SIZE;
+
+  const BatchVariant* var = variant();
+  const int tile = threads * items;
+  P.nfull = P.n / tile;
+  // stage word offsets
+  auto field = [&](int code) {
+    const int width = code & 63;
+    return Field{(code >> 11) * (tile + kColPad), (code >> 6) & 31, width >= 32 ? 0xffffffffu : (1u << width) - 1u};
+  };
+  for (int f = 0; f < P.nfields; ++f) P.at[f].f = field(P.at[f].scode);
+  for (int j = 0; j < P.ndims; ++j) {
+    P.dim[j].key_word *= tile + kColPad;
+    P.dim[j].word *= tile + kColPad;
+  }
+  for (int c = 0; c < P.ncls; ++c) {
+    int qi = 0;  // its first query
+    while (!((P.cls_mask[c][qi / 32] >> (qi % 32)) & 1u)) ++qi;
+    const AQ& A = P.q[qi].a;
+    P.cls[c] = {field(A.a0), field(A.a1), field(A.k0), field(A.k1), A.kmul0, A.kmul1, A.bias,
+                A.total, A.flags & 3, (A.flags >> 5) & 1, ((A.flags >> 3) & 3) > 1 ? 1 : 0};
+  }
+  P.stage_words = stage_cols * (tile + kColPad);
+  auto total_smem = [&](int base, int st) { return (base + 127) / 128 * 128 + st * P.stage_words * 4; };
   P.stages = stages;
   // scalars accumulate in their shared-memory words (kScalarCopies each)
   for (int qi = 0, k = 0; qi < P.nq; ++qi)

@@ -47,3 +47,27 @@ def test_more_group_counts_than_shared_memory_holds(count, smem):
                     preds=[(B.FACT["lo_quantity"], i % 7, 49), (B.FACT["lo_discount"], -3, 13 - i % 5)])
                for i in range(count)]
     _check(5_003, queries, count, smem_group_bytes=smem)
+
+
+@pytest.mark.parametrize("count,values,launch", [
+    (256, 416, {}), (200, 488, {}), (256, 512, {}), (64, 512, dict(threads=512, items_per_thread=4)),
+    (128, 512, dict(threads=512, items_per_thread=4)), (256, 512, dict(threads=512, items_per_thread=4, stages=8))])
+def test_more_tables_than_shared_memory_holds(count, values, launch):
+    """Eight attributes of many values and all nine fact columns: a smaller launch, and tables
+    left in the workspace."""
+    fields = [B.F(M.DIM_COL[k], shift, 9) for k in "SCPD" for shift in (0, 9)]
+    aggs = [(L.MB_AGG_SUB, ["lo_revenue", "lo_supplycost"]), (L.MB_AGG_MUL, ["lo_extendedprice", "lo_discount"]),
+            (L.MB_AGG_SUM, ["lo_quantity"])]
+    rng = np.random.default_rng(count)
+    queries = []
+    for i in range(count):
+        layout = [L.MB_RES_SCALAR, L.MB_RES_CRYSTAL4, L.MB_RES_DENSE][i % 3]
+        keys = [] if layout == L.MB_RES_SCALAR else [(B.F(L.MB_COL_DIM_D, 0, 4), 0, 1), (B.F(L.MB_COL_DIM_S, 4, 3), 0, 16)]
+        preds = [(fields[i % 8], 0, values - 1)]
+        for f in rng.permutation(8)[: int(rng.integers(0, 4))]:
+            lo = int(rng.integers(0, values))
+            preds.append((fields[f], lo, int(rng.integers(lo, values))))
+        op, agg = aggs[i % 3]
+        queries.append(dict(layout=layout, keys=keys, op=op, agg=[B.FACT[a] for a in agg], total=130, dims=i % 16,
+                            preds=preds))
+    _check(6_401, queries, count + values, **launch)
