@@ -275,9 +275,10 @@ class BatchPlan:
 
 
 # launch configurations the batch autotuner tries: consumer threads, rows per thread,
-# stages, shared memory for small group arrays
-BATCH_TUNE_CONFIGS = [(t, i, st, sg) for t, i in ((768, 1), (960, 1), (512, 2), (256, 4))
-                      for st in (2, 3) for sg in (65536, 131072)]
+# stages, shared memory for small group arrays (-1: the default rule, which no size equals).
+# The defaults are among them: 768x2 up to 64 queries, else 960x1, each with 2 stages and -1.
+BATCH_TUNE_CONFIGS = [(t, i, st, sg) for t, i in ((768, 2), (960, 1), (768, 1), (512, 2), (256, 4))
+                      for st in (2, 3) for sg in (-1, 65536, 131072)]
 
 
 def result_buffers(queries: list[Query], device="cuda") -> tuple[torch.Tensor, list[torch.Tensor]]:

@@ -22,6 +22,12 @@ def test_generator_is_seeded_and_spans_selectivities():
     assert {q.groups for q in a} == {1, 175, 7000}
 
 
+def test_the_autotuner_tries_the_default_launches():
+    """768x2 (up to 64 queries), 960x1 and its fallback 768x1, with 2 stages and the default rule
+    for group arrays: a tuned batch is then no slower than an untuned one."""
+    assert {(768, 2, 2, -1), (960, 1, 2, -1), (768, 1, 2, -1)} <= set(B.BATCH_TUNE_CONFIGS)
+
+
 def test_descriptor_fields_fit_the_encoding():
     for q in B.generate_queries(30, seed=1):
         c = q.to_c(type("R", (), {"data_ptr": lambda self: 4096})())
