@@ -559,7 +559,7 @@ __global__ void __launch_bounds__((NCW + 1) * 32, 1) batch_kernel(const __grid_c
               if (h < 0)
                 bad_probe = true;
               else if (want)
-                word[r][j] = __ldg(D.pat + h);
+                word[r][j] = static_cast<unsigned>(ld_word(reinterpret_cast<const int*>(D.pat) + h));
             }
           }
         };
@@ -731,7 +731,7 @@ __global__ void __launch_bounds__((NCW + 1) * 32, 1) batch_kernel(const __grid_c
             bad_probe = true;
             continue;
           }
-          dimw[d] = static_cast<int>(__ldg(P.dim[j].pat + h));
+          dimw[d] = ld_word(reinterpret_cast<const int*>(P.dim[j].pat) + h);
           pr |= (static_cast<unsigned>(dimw[d]) >> 31) << d;
         }
         auto get = [&](int code) {

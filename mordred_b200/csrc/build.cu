@@ -45,7 +45,7 @@ struct BuildPlan {
 __device__ __forceinline__ long long build_row_index(const BuildPlan& B, long long r, int* seg_out) {
   if (B.rows != nullptr) {
     // a listed dimension row: the physical row, through its own segment's slot
-    const long long d = __ldg(B.rows + r);
+    const long long d = ld_word(B.rows + r);
     if (B.gpu_cache == nullptr) {
       *seg_out = 0;
       return d;
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(kBuildThreads) build_kernel(const __grid_const
     const int v = B.val != nullptr ? build_load(B, B.val, seg, idx) : 0;
     // the row's position in the table (segment * segment_size + in-segment offset, or the
     // listed row)
-    const long long rowid = B.rows != nullptr       ? static_cast<long long>(__ldg(B.rows + r))
+    const long long rowid = B.rows != nullptr       ? static_cast<long long>(ld_word(B.rows + r))
                             : B.gpu_cache == nullptr ? B.start_offset + r
                                                      : (static_cast<long long>(seg) << B.seg_shift) + idx;
     build_row(B, rowid, key, v, R);

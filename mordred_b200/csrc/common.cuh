@@ -109,8 +109,24 @@ __device__ __forceinline__ int4 lds128(const int* p) {
 }
 
 // Read-only 8-byte hash-table slot through the non-coherent path.
-__device__ __forceinline__ unsigned long long ldg_u64(const int* p) {
-  return __ldg(reinterpret_cast<const unsigned long long*>(p));
+// Words that a kernel before this one in the stream may have written: hash tables, presence
+// bitmaps, attribute tables, offset lists. A dependent launch (below) may begin while that kernel
+// still runs, so they are plain loads — ld.global.nc and __ldg are for memory that nothing writes
+// from the launch on (fact and dimension columns, cache slots).
+__device__ __forceinline__ int ld_word(const int* p) {
+  int v;
+  asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ unsigned long long ld_word2(const int* p) {
+  unsigned long long v;
+  asm volatile("ld.global.b64 %0, [%1];" : "=l"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int4 ld_word4(const int* p) {
+  int4 v;
+  asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
 }
 
 // *sum += v (sign-extended), a 64-bit sum in shared memory, as two 32-bit atomics: the low

@@ -86,11 +86,11 @@ struct __align__(16) SelWarp {
 // The word(s) of slot h (>= 0): present, and the probe's output.
 __device__ __forceinline__ bool sel_lookup(const int* ht, int layout, int h, int& out) {
   if (layout == MB_HT_KEY_VAL) {
-    const unsigned long long s = ldg_u64(ht + 2ll * h);
+    const unsigned long long s = ld_word2(ht + 2ll * h);
     out = static_cast<int>(s >> 32);
     return s != 0;
   }
-  const int w = __ldg(layout == MB_HT_KEY ? ht + h : ht + 2ll * h + 1);
+  const int w = ld_word(layout == MB_HT_KEY ? ht + h : ht + 2ll * h + 1);
   out = layout == MB_HT_KEY ? 0 : w - 1;
   return w != 0;
 }
@@ -205,9 +205,9 @@ __global__ void __launch_bounds__(kSelMaxWarps * 32, 1) select_slices_kernel(con
     const int slots = P.pslots[0], layout = P.playout[0];
     auto present = [&](int h) {
       if (h >= slots) return false;
-      return layout == MB_HT_KEY       ? __ldg(ht + h) != 0
-             : layout == MB_HT_VAL_OFF ? __ldg(ht + 2ll * h + 1) != 0
-                                       : ldg_u64(ht + 2ll * h) != 0ull;
+      return layout == MB_HT_KEY       ? ld_word(ht + h) != 0
+             : layout == MB_HT_VAL_OFF ? ld_word(ht + 2ll * h + 1) != 0
+                                       : ld_word2(ht + 2ll * h) != 0ull;
     };
     const bool pairs = layout != MB_HT_KEY && (reinterpret_cast<uintptr_t>(ht) & 15u) == 0;
 #pragma unroll 8
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(kSelMaxWarps * 32, 1) select_slices_kernel(con
       const int h = word * 32 + 2 * lane;
       bool even, odd;
       if (pairs && h + 1 < slots) {
-        const int4 t = __ldg(reinterpret_cast<const int4*>(ht + 2ll * h));
+        const int4 t = ld_word4(ht + 2ll * h);
         even = layout == MB_HT_VAL_OFF ? t.y != 0 : (t.x | t.y) != 0;
         odd = layout == MB_HT_VAL_OFF ? t.w != 0 : (t.z | t.w) != 0;
       } else {
@@ -468,13 +468,13 @@ __global__ void __launch_bounds__(256) select_kernel(const __grid_constant__ Sel
         }
         const int* ht = P.pht[p];
         if (P.playout[p] == MB_HT_KEY) {
-          ok = __ldg(ht + h) != 0;
+          ok = ld_word(ht + h) != 0;
         } else if (P.playout[p] == MB_HT_VAL_OFF) {
-          const int w = __ldg(ht + 2ll * h + 1);
+          const int w = ld_word(ht + 2ll * h + 1);
           ok = w != 0;
           outv[p] = w - 1;
         } else {
-          const unsigned long long s = ldg_u64(ht + 2ll * h);
+          const unsigned long long s = ld_word2(ht + 2ll * h);
           ok = s != 0;
           outv[p] = static_cast<int>(s >> 32);
         }

@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kListThreads, kListCtas) list_kernel(const __g
       if (k < P.n) {
         sel |= 1u << i;
         if (P.rows) {
-          idx[i] = __ldg(P.rows + k);
+          idx[i] = ld_word(P.rows + k);
         } else {
           idx[i] = static_cast<Index>(SEG ? k & ((1ll << P.seg_shift) - 1) : k);
           if (SEG)
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(kListThreads, kListCtas) list_kernel(const __g
         if (P.p_layout[p] == MB_HT_PASS) {
 #pragma unroll
           for (int i = 0; i < R; ++i)
-            if ((sel >> i) & 1u) gv[p][i] = __ldg(P.p_key[p] + base + static_cast<long long>(i) * kListThreads);
+            if ((sel >> i) & 1u) gv[p][i] = ld_word(P.p_key[p] + base + static_cast<long long>(i) * kListThreads);
         } else {
           load(P.p_key[p], sel, gv[p]);
         }
@@ -207,10 +207,10 @@ __global__ void __launch_bounds__(kListThreads, kListCtas) list_kernel(const __g
         const unsigned of = sel & ~range_bad[p];
         if (layout == MB_HT_KEY) {
 #pragma unroll
-          for (int i = 0; i < R; ++i) sv[p][i] = (of >> i) & 1u ? static_cast<unsigned>(__ldg(ht + h[i])) : 0u;
+          for (int i = 0; i < R; ++i) sv[p][i] = (of >> i) & 1u ? static_cast<unsigned>(ld_word(ht + h[i])) : 0u;
         } else {
 #pragma unroll
-          for (int i = 0; i < R; ++i) sv[p][i] = (of >> i) & 1u ? ldg_u64(ht + 2ll * h[i]) : 0ull;
+          for (int i = 0; i < R; ++i) sv[p][i] = (of >> i) & 1u ? ld_word2(ht + 2ll * h[i]) : 0ull;
         }
       }
 #pragma unroll

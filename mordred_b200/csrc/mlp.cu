@@ -8,6 +8,9 @@
 // W3[64][2], b3[2]; W[i][j] is input i -> unit j. SIMT fp32 on purpose: the planner's
 // predictions and gradients keep fp32 products and sums (a tensor-core split would not),
 // so the roofline is the fp32 FMA rate, 148 SMs x 128 lanes x 2 x 1.965 GHz = 74.4 TFLOP/s.
+// The kernels' pointers are not __restrict__: parameters and gradients are written by the kernel
+// before, which may still run when a dependent launch begins, and const __restrict__ would have
+// them read by non-coherent loads.
 #include <cmath>
 
 #include "common.cuh"
@@ -103,9 +106,8 @@ __device__ __forceinline__ void fwd_layer(const float* in, const float* w, const
 }
 
 template <int S>
-__global__ void __launch_bounds__(kFwdWarps * 32, 1) mlp_forward_kernel(const float* __restrict__ params,
-                                                                       const float* __restrict__ x, int batch,
-                                                                       float* __restrict__ y) {
+__global__ void __launch_bounds__(kFwdWarps * 32, 1) mlp_forward_kernel(const float* params, const float* x,
+                                                                       int batch, float* y) {
   extern __shared__ __align__(16) unsigned char raw[];
   FwdSmem<S>& s = *reinterpret_cast<FwdSmem<S>*>(raw);
   constexpr int kTile = 8 * S;  // samples per warp
@@ -259,10 +261,9 @@ struct BwdSmem {
 };
 
 template <int T>
-__global__ void __launch_bounds__(kBwdThreads) mlp_backward_kernel(const float* __restrict__ params,
-                                                                   const float* __restrict__ x,
-                                                                   const float* __restrict__ target, int batch,
-                                                                   float* __restrict__ grads, float* loss_sum) {
+__global__ void __launch_bounds__(kBwdThreads) mlp_backward_kernel(const float* params, const float* x,
+                                                                   const float* target, int batch, float* grads,
+                                                                   float* loss_sum) {
   extern __shared__ __align__(16) unsigned char raw[];
   BwdSmem<T>& s = *reinterpret_cast<BwdSmem<T>*>(raw);
   constexpr int NS = T / 4;  // samples a thread computes in each layer
@@ -407,9 +408,8 @@ __global__ void __launch_bounds__(kBwdThreads) mlp_backward_kernel(const float* 
   }
 }
 
-__global__ void mlp_adam_kernel(float* __restrict__ params, const float* __restrict__ grads, float* __restrict__ m,
-                                float* __restrict__ v, int n, float lr, float beta1, float beta2, float eps,
-                                float bc1, float bc2, float weight_decay) {
+__global__ void mlp_adam_kernel(float* params, const float* grads, float* m, float* v, int n, float lr, float beta1,
+                                float beta2, float eps, float bc1, float bc2, float weight_decay) {
   allow_dependent();
   wait_for_predecessor();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {

@@ -72,40 +72,36 @@ __device__ __forceinline__ uint32_t mirror_word(const StarPlan& P, int p, int re
     const int s0 = rel * 32;
     if (P.p_layout[p] == MB_HT_KEY) {
       if (s0 + 32 <= slots && aligned16_dev(ht)) {
-        const int4* src = reinterpret_cast<const int4*>(ht + s0);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const int4 q = __ldg(src + j);
+          const int4 q = ld_word4(ht + s0 + 4 * j);
           w |= ((q.x != 0 ? 1u : 0u) << (4 * j)) | ((q.y != 0 ? 1u : 0u) << (4 * j + 1)) |
                ((q.z != 0 ? 1u : 0u) << (4 * j + 2)) | ((q.w != 0 ? 1u : 0u) << (4 * j + 3));
         }
       } else {
-        for (int j = 0; j < 32 && s0 + j < slots; ++j) w |= (__ldg(ht + s0 + j) != 0 ? 1u : 0u) << j;
+        for (int j = 0; j < 32 && s0 + j < slots; ++j) w |= (ld_word(ht + s0 + j) != 0 ? 1u : 0u) << j;
       }
     } else {
-      const unsigned long long* t8 = reinterpret_cast<const unsigned long long*>(ht);
       if (s0 + 32 <= slots && aligned16_dev(ht)) {
-        const ulonglong2* src = reinterpret_cast<const ulonglong2*>(t8 + s0);
 #pragma unroll 4
         for (int j = 0; j < 16; ++j) {
-          const ulonglong2 q = __ldg(src + j);
-          w |= ((q.x != 0ull ? 1u : 0u) << (2 * j)) | ((q.y != 0ull ? 1u : 0u) << (2 * j + 1));
+          const int4 q = ld_word4(ht + 2ll * (s0 + 2 * j));
+          w |= (((q.x | q.y) != 0 ? 1u : 0u) << (2 * j)) | (((q.z | q.w) != 0 ? 1u : 0u) << (2 * j + 1));
         }
       } else {
-        for (int j = 0; j < 32 && s0 + j < slots; ++j) w |= (__ldg(t8 + s0 + j) != 0ull ? 1u : 0u) << j;
+        for (int j = 0; j < 32 && s0 + j < slots; ++j) w |= (ld_word2(ht + 2ll * (s0 + j)) != 0ull ? 1u : 0u) << j;
       }
     }
     return w;
   }
   // payload codes: 0 absent, 1..14 payload - min + 1, 15 present with another payload
   const int s0 = rel * 8;
-  const unsigned long long* t8 = reinterpret_cast<const unsigned long long*>(ht);
   const bool hi = P.p_layout[p] == MB_HT_KEY_VAL;
   const unsigned mn = static_cast<unsigned>(P.mir_min[p]);
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     if (s0 + j >= slots) break;
-    const unsigned long long v = __ldg(t8 + s0 + j);
+    const unsigned long long v = ld_word2(ht + 2ll * (s0 + j));
     if (v == 0ull) continue;
     const unsigned pay = hi ? static_cast<unsigned>(v >> 32) : static_cast<unsigned>(v);
     const unsigned d = pay - mn;
@@ -313,9 +309,9 @@ __device__ __forceinline__ void probe_round(const StarPlan& P, const L& ld, uint
         else if (bm != nullptr && !((bm[h >> 5] >> (h & 31)) & 1u))
           absent[q] |= 1u << i;
         else if (layout == MB_HT_KEY)
-          sv[q][i] = bm != nullptr ? 1ull : static_cast<unsigned long long>(static_cast<unsigned>(__ldg(ht + h)));
+          sv[q][i] = bm != nullptr ? 1ull : static_cast<unsigned long long>(static_cast<unsigned>(ld_word(ht + h)));
         else
-          sv[q][i] = ldg_u64(ht + 2 * h);
+          sv[q][i] = ld_word2(ht + 2 * h);
       }
     }
   }
@@ -595,9 +591,9 @@ __device__ __forceinline__ void sparse_rows_mir(const StarPlan& P, const L& ld, 
           sv[q][i] = (ld_dsmem_u32(share + 4u * static_cast<uint32_t>(gw & smask), static_cast<uint32_t>(gw) >> P.mir_shift) >>
                       (4 * (h & 7))) & 15u;
         } else if (layout == MB_HT_KEY) {
-          sv[q][i] = bm != nullptr ? 1ull : static_cast<unsigned long long>(static_cast<unsigned>(__ldg(ht + h)));
+          sv[q][i] = bm != nullptr ? 1ull : static_cast<unsigned long long>(static_cast<unsigned>(ld_word(ht + h)));
         } else {
-          sv[q][i] = ldg_u64(ht + 2 * h);
+          sv[q][i] = ld_word2(ht + 2 * h);
         }
       }
     }
@@ -643,7 +639,7 @@ __device__ __forceinline__ void sparse_rows_mir(const StarPlan& P, const L& ld, 
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
       if (!(fetch[q] & sel & (1u << i))) continue;
-      const unsigned long long raw = ldg_u64(ht + 2 * pht_slot(v[i], P.p_slots[p], P.p_kmin[p]));
+      const unsigned long long raw = ld_word2(ht + 2 * pht_slot(v[i], P.p_slots[p], P.p_kmin[p]));
       gv[q][i] = hi ? static_cast<int>(raw >> 32) : static_cast<int>(static_cast<unsigned>(raw));
     }
   }
@@ -788,29 +784,29 @@ __global__ void __launch_bounds__((NCW + 1) * 32, star_min_ctas(NCW)) star_kerne
     uint32_t* bm = reinterpret_cast<uint32_t*>(smem + P.p_bm_off[p]);
     const int words = P.p_bm_words[p];
     if (P.p_presence[p] != nullptr) {
-      for (int w = tid; w < words; w += NWARPS * 32) bm[w] = __ldg(P.p_presence[p] + w);
+      for (int w = tid; w < words; w += NWARPS * 32) bm[w] = static_cast<uint32_t>(ld_word(reinterpret_cast<const int*>(P.p_presence[p]) + w));
     } else if (P.p_layout[p] != MB_HT_KEY) {
       // derive presence from a table with 8-byte slots: slot s is present when nonzero
       const int slots = P.p_slots[p];
-      const unsigned long long* ht = reinterpret_cast<const unsigned long long*>(P.p_ht[p]);
+      const int* ht = P.p_ht[p];
       const bool vec = aligned16_dev(ht);
       for (int w = tid; w < words; w += NWARPS * 32) {
         uint32_t word = 0;
         if (vec && (w + 1) * 32 <= slots) {
           // four 16-byte loads (8 slots) in flight at a time: few registers, so the set-up
           // does not raise the kernel's register count
-          const ulonglong2* src = reinterpret_cast<const ulonglong2*>(ht + w * 32);
 #pragma unroll 1
           for (int j0 = 0; j0 < 16; j0 += 4) {
-            ulonglong2 q[4];
+            int4 q[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) q[j] = __ldg(src + j0 + j);
+            for (int j = 0; j < 4; ++j) q[j] = ld_word4(ht + w * 64 + 4 * (j0 + j));
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-              word |= ((q[j].x != 0ull ? 1u : 0u) << (2 * (j0 + j))) | ((q[j].y != 0ull ? 1u : 0u) << (2 * (j0 + j) + 1));
+              word |= (((q[j].x | q[j].y) != 0 ? 1u : 0u) << (2 * (j0 + j))) |
+                      (((q[j].z | q[j].w) != 0 ? 1u : 0u) << (2 * (j0 + j) + 1));
           }
         } else {
-          for (int j = 0; j < 32 && w * 32 + j < slots; ++j) word |= (__ldg(ht + w * 32 + j) != 0ull ? 1u : 0u) << j;
+          for (int j = 0; j < 32 && w * 32 + j < slots; ++j) word |= (ld_word2(ht + 2 * (w * 32 + j)) != 0ull ? 1u : 0u) << j;
         }
         bm[w] = word;
       }
@@ -825,13 +821,13 @@ __global__ void __launch_bounds__((NCW + 1) * 32, star_min_ctas(NCW)) star_kerne
         if (vec && (w + 1) * 32 <= slots) {
           int4 q[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) q[j] = __ldg(reinterpret_cast<const int4*>(ht + w * 32) + j);
+          for (int j = 0; j < 8; ++j) q[j] = ld_word4(ht + w * 32 + 4 * j);
 #pragma unroll
           for (int j = 0; j < 8; ++j)
             word |= ((q[j].x != 0 ? 1u : 0u) << (4 * j)) | ((q[j].y != 0 ? 1u : 0u) << (4 * j + 1)) |
                     ((q[j].z != 0 ? 1u : 0u) << (4 * j + 2)) | ((q[j].w != 0 ? 1u : 0u) << (4 * j + 3));
         } else {
-          for (int j = 0; j < 32 && w * 32 + j < slots; ++j) word |= (__ldg(ht + w * 32 + j) != 0 ? 1u : 0u) << j;
+          for (int j = 0; j < 32 && w * 32 + j < slots; ++j) word |= (ld_word(ht + w * 32 + j) != 0 ? 1u : 0u) << j;
         }
         bm[w] = word;
       }

@@ -55,8 +55,8 @@ __device__ __forceinline__ void ring_word(const int* ht, bool key_layout, int h,
       "{\n\t.reg .pred k, v;\n\t"
       "setp.eq.u32 k, %4, 1;\n\t"
       "setp.eq.u32 v, %4, 2;\n\t"
-      "@k ld.global.nc.u32 %0, [%2];\n\t"
-      "@v ld.global.nc.v2.u32 {%0, %1}, [%3];\n\t}"
+      "@k ld.global.u32 %0, [%2];\n\t"
+      "@v ld.global.v2.u32 {%0, %1}, [%3];\n\t}"
       : "+r"(lo), "+r"(hi)
       : "l"(ht + h), "l"(ht + 2ll * h), "r"(!on ? 0u : key_layout ? 1u : 2u));
 }
@@ -103,7 +103,8 @@ __device__ __forceinline__ void ring_stage_bitmap(const StarPlan& P, int p, uint
     const int given = (slots + 31) / 32;
     const uint32_t tail = slots % 32 != 0 ? (1u << (slots % 32)) - 1u : kFull;
     for (int w = warp * 32 + lane; w < words; w += nwarps * 32) {
-      uint32_t v = w < given ? __ldg(P.p_presence[p] + w) : 0u;
+      uint32_t v = 0u;
+      if (w < given) v = static_cast<uint32_t>(ld_word(reinterpret_cast<const int*>(P.p_presence[p]) + w));
       if (w == given - 1) v &= tail;
       bm[w] = __brev(v);
     }
@@ -118,12 +119,12 @@ __device__ __forceinline__ void ring_stage_bitmap(const StarPlan& P, int p, uint
       const int h = w0 * 32 + 4 * lane;
       int4 t = make_int4(0, 0, 0, 0);
       if (aligned && h + 3 < slots) {
-        t = __ldg(reinterpret_cast<const int4*>(ht + h));
+        t = ld_word4(ht + h);
       } else {
-        if (h < slots) t.x = __ldg(ht + h);
-        if (h + 1 < slots) t.y = __ldg(ht + h + 1);
-        if (h + 2 < slots) t.z = __ldg(ht + h + 2);
-        if (h + 3 < slots) t.w = __ldg(ht + h + 3);
+        if (h < slots) t.x = ld_word(ht + h);
+        if (h + 1 < slots) t.y = ld_word(ht + h + 1);
+        if (h + 2 < slots) t.z = ld_word(ht + h + 2);
+        if (h + 3 < slots) t.w = ld_word(ht + h + 3);
       }
       // lane l's nibble in slot order, then eight lanes' nibbles into a word
       uint32_t nib = (t.x != 0 ? 8u : 0u) | (t.y != 0 ? 4u : 0u) | (t.z != 0 ? 2u : 0u) | (t.w != 0 ? 1u : 0u);
@@ -135,18 +136,19 @@ __device__ __forceinline__ void ring_stage_bitmap(const StarPlan& P, int p, uint
     }
   } else {
     // 64 slots of 8 bytes a warp step, two a lane, sixteen lanes' pairs into a word
-    const unsigned long long* t8 = reinterpret_cast<const unsigned long long*>(ht);
 #pragma unroll 4
     for (int w0 = 2 * warp; w0 < words; w0 += 2 * nwarps) {
       const int h = w0 * 32 + 2 * lane;
-      ulonglong2 t = make_ulonglong2(0ull, 0ull);
+      bool even = false, odd = false;
       if (aligned && h + 1 < slots) {
-        t = __ldg(reinterpret_cast<const ulonglong2*>(t8 + h));
+        const int4 t = ld_word4(ht + 2ll * h);
+        even = (t.x | t.y) != 0;
+        odd = (t.z | t.w) != 0;
       } else {
-        if (h < slots) t.x = __ldg(t8 + h);
-        if (h + 1 < slots) t.y = __ldg(t8 + h + 1);
+        if (h < slots) even = ld_word2(ht + 2ll * h) != 0ull;
+        if (h + 1 < slots) odd = ld_word2(ht + 2ll * h + 2) != 0ull;
       }
-      uint32_t word = ((t.x != 0ull ? 2u : 0u) | (t.y != 0ull ? 1u : 0u)) << (30 - 2 * (lane & 15));
+      uint32_t word = ((even ? 2u : 0u) | (odd ? 1u : 0u)) << (30 - 2 * (lane & 15));
 #pragma unroll
       for (int o = 1; o < 16; o <<= 1) word |= __shfl_xor_sync(kFull, word, o);
       if ((lane & 15) == 0 && w0 + (lane >> 4) < words) bm[w0 + (lane >> 4)] = word;
