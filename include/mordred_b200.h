@@ -172,7 +172,8 @@ int mb_build_pht(const int* filter_col, int filter_mode, int c1, int c2,
 
 /* The tables of a query in two launches: clears every table (int[num_slots], with dim_val
  * int[2 * num_slots]), its presence bitmap and `zero` (zero_words 32-bit words, optional: the
- * query's result), then builds each as mb_build_pht does. */
+ * query's result), then builds each as mb_build_pht does. Builds that write the same memory run
+ * one after the other, in the order given, in a launch more each. */
 #define MB_MAX_TABLE_BUILDS 8
 typedef struct mb_table_build {
   const int* filter_col;

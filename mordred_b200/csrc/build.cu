@@ -268,7 +268,8 @@ extern "C" int mb_build_tables(const mb_table_build* builds, int num_builds, int
                                mb_stream_t stream) {
   if (num_builds < 0 || num_builds > MB_MAX_TABLE_BUILDS || (num_builds > 0 && builds == nullptr)) return MB_ERR_ARG;
   if (zero_words < 0 || (zero_words > 0 && zero == nullptr)) return MB_ERR_ARG;
-  BuildMany M = {};
+  BuildPlan plan[MB_MAX_TABLE_BUILDS] = {};
+  int count = 0;
   ZeroMany Z = {};
   auto clear = [&](void* p, long long words) {
     if (words == 0) return;
@@ -286,7 +287,7 @@ extern "C" int mb_build_tables(const mb_table_build* builds, int num_builds, int
     clear(b.ht, (b.dim_val != nullptr ? 2ll : 1ll) * b.num_slots);
     if (b.presence != nullptr) clear(b.presence, (b.num_slots + 31ll) / 32);
     if (b.num_tuples == 0) continue;
-    BuildPlan& B = M.b[M.count];
+    BuildPlan& B = plan[count++];
     B.filter = b.filter_col;
     B.mode = b.filter_mode;
     B.c1 = b.c1;
@@ -299,14 +300,10 @@ extern "C" int mb_build_tables(const mb_table_build* builds, int num_builds, int
     B.kmin = b.key_min;
     B.layout = b.dim_val != nullptr ? MB_HT_KEY_VAL : MB_HT_KEY;
     B.presence = b.presence;
-    const long long per_block = static_cast<long long>(kBuildThreads) * kBuildItems;
-    M.first[M.count + 1] = M.first[M.count] + static_cast<int>((B.n + per_block - 1) / per_block);
-    ++M.count;
   }
   int err = MB_OK;
   DeviceState* ds = current_device_state(&err);
   if (ds == nullptr) return err;
-  for (int t = 0; t < M.count; ++t) M.b[t].status = ds->status;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (Z.count > 0) {
     long long most = 0;
@@ -318,7 +315,30 @@ extern "C" int mb_build_tables(const mb_table_build* builds, int num_builds, int
       return MB_ERR_LAUNCH;
     note_launches(1);
   }
-  if (M.count > 0) {
+  // all of them together, but a build into memory that an earlier one writes after that one
+  auto shares = [](const BuildPlan& x, const BuildPlan& y) {
+    auto meet = [](const void* p, long long pw, const void* q, long long qw) {  // of pw and qw words
+      const uintptr_t a = reinterpret_cast<uintptr_t>(p), b = reinterpret_cast<uintptr_t>(q);
+      return a != 0 && b != 0 && a < b + 4 * static_cast<uintptr_t>(qw) && b < a + 4 * static_cast<uintptr_t>(pw);
+    };
+    const long long xt = (x.layout == MB_HT_KEY ? 1ll : 2ll) * x.slots, xb = (x.slots + 31ll) / 32;
+    const long long yt = (y.layout == MB_HT_KEY ? 1ll : 2ll) * y.slots, yb = (y.slots + 31ll) / 32;
+    return meet(x.ht, xt, y.ht, yt) || meet(x.ht, xt, y.presence, yb) || meet(x.presence, xb, y.ht, yt) ||
+           meet(x.presence, xb, y.presence, yb);
+  };
+  for (int t = 0; t < count;) {
+    BuildMany M = {};
+    for (; t < count; ++t) {
+      bool after = false;
+      for (int o = 0; o < M.count; ++o) after = after || shares(plan[t], M.b[o]);
+      if (after) break;
+      BuildPlan& B = M.b[M.count];
+      B = plan[t];
+      B.status = ds->status;
+      const long long per_block = static_cast<long long>(kBuildThreads) * kBuildItems;
+      M.first[M.count + 1] = M.first[M.count] + static_cast<int>((B.n + per_block - 1) / per_block);
+      ++M.count;
+    }
     if (launch_dependent(build_many_kernel, M.first[M.count], kBuildThreads, 0, st, M) != cudaSuccess)
       return MB_ERR_LAUNCH;
     note_launches(1);

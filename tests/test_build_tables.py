@@ -61,6 +61,35 @@ def test_tables_together(n, shift):
     assert L.device_status(0) == 0
 
 
+@pytest.mark.parametrize("n", [5, 300_003])
+def test_builds_into_one_table_keep_their_order(n):
+    """Three builds into one table (or its bitmap alone), a fourth into another between them: rows
+    of a later build replace the payloads of an earlier one's, and the first key stays."""
+    rng = np.random.default_rng(n)
+    slots = 2 * n + 3
+    dims = [_dimension(rng, n, 1) for _ in range(4)]
+    tables = [torch.full((2 * slots,), 7, dtype=torch.int32, device="cuda") for _ in range(2)]
+    bits = torch.full(((slots + 31) // 32,), -1, dtype=torch.int32, device="cuda")
+    cols = [[_dev(d[k]) for k in ("flt", "key", "val")] for d in dims]
+    arr = (L.MbTableBuild * 4)()
+    into = [0, 1, 0, 0]
+    for b, c, d, k in zip(arr, cols, dims, into):
+        b.filter_col, b.dim_key, b.dim_val = (ssb._p(x) for x in c)
+        b.filter_mode, b.c1, b.c2 = d["mode"], 1, 3
+        b.num_tuples, b.ht, b.num_slots, b.key_min = n, tables[k].data_ptr(), slots, d["kmin"]
+        b.presence = bits.data_ptr() if k == 0 else None
+    L.call("mb_build_tables", arr, 4, None, 0, ssb._stream())
+    torch.cuda.synchronize()
+    ref = [np.zeros(2 * slots, np.int32) for _ in range(2)]
+    for d, k in zip(dims, into):
+        O.build_ht(d["flt"], d["mode"], 1, 3, d["key"], d["val"], ref[k], slots, d["kmin"], L.MB_HT_KEY_VAL)
+    for t, r in zip(tables, ref):
+        assert np.array_equal(t.cpu().numpy(), r)
+    packed = np.zeros(bits.numel() * 32, np.uint8)
+    packed[:slots] = ref[0].reshape(-1, 2).any(1)
+    assert np.array_equal(bits.cpu().numpy(), np.packbits(packed, bitorder="little").view(np.int32))
+
+
 @pytest.mark.parametrize("n", [1, 9, 2_049, 300_003])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_single_build_of_columns(n, shift):
