@@ -198,7 +198,9 @@ inline cudaError_t launch_dependent(void (*fn)(Params...), int grid, int block, 
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, fn, static_cast<Params>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, fn, static_cast<Params>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();  // reported by the caller: not for a later call to find
+  return e;
 }
 
 inline int cuda_status(cudaError_t e) { return e == cudaSuccess ? MB_OK : MB_ERR_CUDA; }

@@ -68,3 +68,26 @@ def test_training_steps_in_a_row():
         ends.append((params, y))
     assert torch.equal(ends[0][0], ends[1][0]) and torch.equal(ends[0][1], ends[1][1])
     assert np.isfinite(ends[0][1].cpu().numpy()).all()
+
+
+def test_a_launch_that_fails_leaves_nothing_behind():
+    """A launch on the legacy stream while another stream captures is refused by the runtime. The
+    call says so; the next one, of a kernel that looks the last error up, is not refused for it."""
+    import ctypes as C
+    p = torch.zeros(64, device="cuda")
+    key = torch.arange(1, 9, dtype=torch.int32, device="cuda")
+    words = torch.zeros(16, dtype=torch.int32, device="cuda")
+    adam = (p.data_ptr(), p.data_ptr(), p.data_ptr(), p.data_ptr(), 64, 1e-3, 0.9, 0.999, 1e-8, 1, 0.0, None)
+    torch.cuda.synchronize()
+    runtime = C.CDLL("libcudart.so.12")
+    stream, graph = C.c_void_p(), C.c_void_p()
+    assert runtime.cudaStreamCreate(C.byref(stream)) == 0
+    assert runtime.cudaStreamBeginCapture(stream, 0) == 0  # global mode
+    refused = L.lib().mb_mlp_adam(*adam)
+    runtime.cudaStreamEndCapture(stream, C.byref(graph))
+    runtime.cudaStreamDestroy(stream)
+    runtime.cudaGetLastError()
+    assert refused != L.MB_OK
+    L.call("mb_pat_build", key.data_ptr(), 8, 0, 16, None, 0, None, 0, None, 0, words.data_ptr(), None)
+    torch.cuda.synchronize()
+    assert int((words != 0).sum()) == 8
