@@ -69,8 +69,9 @@ struct StarPlan {
   int sparse_p0;                  // first probe of the sparse phase: the leading bitmap-tested
                                   // probes whose payload is not needed stop before it, the
                                   // others are probed again there for their payload
-  unsigned dense_bias;            // group terms (0 - min_val) * unique_val of probes < sparse_p0
-  int sp_ord[MB_MAX_PROBES];      // tiled path: probe visited at sparse position q (the first
+                                  // (star_ring.cu: how many bitmap probes are settled, of all)
+  unsigned dense_bias;            // group terms (0 - min_val) * unique_val of the settled probes
+  int sp_ord[MB_MAX_PROBES];      // probe visited at sparse position q (the first
                                   // probe that can drop rows leads; the dense phase settled the
                                   // probes it passes, which are read only for their payloads)
   int p_col[MB_MAX_PROBES];

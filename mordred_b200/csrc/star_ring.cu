@@ -169,7 +169,8 @@ __global__ void __launch_bounds__(kRingMaxWarps * 32, 1) star_ring_kernel(const 
   int* stage = reinterpret_cast<int*>(mine + sizeof(RingWarp));
   unsigned long long* s_sum = reinterpret_cast<unsigned long long*>(smem + P.smem_groups_off);
   uint32_t* s_touch = reinterpret_cast<uint32_t*>(smem + P.smem_groups_off + 8 * P.total_val);
-  const int nf = NFC >= 0 ? NFC : P.nf, nd = NDC >= 0 ? NDC : P.n_dense, ns = P.np - P.sparse_p0;
+  const int nf = NFC >= 0 ? NFC : P.nf, nd = NDC >= 0 ? NDC : P.n_dense;
+  const int ns = P.np - P.sparse_p0;  // sparse_p0: bitmap probes settled by their bit
   const unsigned bias = static_cast<unsigned>(P.group_bias) + P.dense_bias;
   const bool two_cols = P.agg_op == MB_AGG_SUB || P.agg_op == MB_AGG_MUL;
   // the aggregate columns are gathered with the remaining keys, unless two or more tables can
@@ -553,7 +554,7 @@ int launch_ring(StarPlan& P, int group_mode, const DeviceState& ds, cudaStream_t
   P.smem_groups_off = off;
   if (P.gmode == kGroupSmem) off += (8 * P.total_val + 4 * ((P.total_val + 31) / 32) + 15) / 16 * 16;
   int bm_total = 0;
-  bool settled = true;
+  int read[MB_MAX_PROBES], nread = 0;  // bitmap probes whose payload somebody reads
   for (int p = 0; p < P.np; ++p) {
     P.p_bm_off[p] = -1;
     P.p_bm_words[p] = 0;
@@ -566,21 +567,26 @@ int launch_ring(StarPlan& P, int group_mode, const DeviceState& ds, cudaStream_t
     P.p_bm_words[p] = bytes / 4;
     bm_total += (bytes + 15) / 16 * 16;
     P.n_dense = p + 1;
-    // one whose payload nobody reads is settled by its bit: its group term is a constant
-    const bool free = P.p_layout[p] == MB_HT_KEY || (P.p_mul[p] == 0 && P.p_res_slot[p] < 0);
-    settled = settled && free;
-    if (settled) {
-      P.sparse_p0 = p + 1;
+    // one whose payload nobody reads is settled by its bit, wherever it stands: its group term is
+    // a constant (24,000,000 rows, a date table before a 40,000-slot key table and a third probe:
+    // 82 us with a fifth of the rows kept by each and 607 with all of them kept when the key table
+    // was looked up again, now 79 and 414; the tile kernels 182 and 514)
+    if (P.p_layout[p] == MB_HT_KEY || (P.p_mul[p] == 0 && P.p_res_slot[p] < 0)) {
+      ++P.sparse_p0;
       P.dense_bias += (0u - static_cast<unsigned>(P.p_min[p])) * static_cast<unsigned>(P.p_mul[p]);
+    } else {
+      read[nread++] = p;
     }
   }
   off = (off + bm_total + 127) / 128 * 128;
   P.smem_list_off = off;
-  // visiting order: chain order, except that the first probe the bitmaps did not settle leads
-  // (the settled ones are read for their payloads only); it runs before the ring
-  const int ns = P.np - P.sparse_p0, lead = P.n_dense - P.sparse_p0;
-  const bool key = lead < ns;
-  for (int q = 0; q < ns; ++q) P.sp_ord[q] = P.sparse_p0 + (!key ? q : q == 0 ? lead : q <= lead ? q - 1 : q);
+  // visiting order of the others: chain order, except that the first probe without a bitmap
+  // leads (the bitmap probes are read for their payloads only); it runs before the ring
+  const bool key = P.n_dense < P.np;
+  int ns = 0;
+  if (key) P.sp_ord[ns++] = P.n_dense;
+  for (int i = 0; i < nread; ++i) P.sp_ord[ns++] = read[i];
+  for (int p = P.n_dense + 1; p < P.np; ++p) P.sp_ord[ns++] = p;
   // staged columns
   P.r_nst = 0;
   auto staged = [&](int c) {

@@ -2,6 +2,8 @@
 every table layout for the bitmap-decided, the first and the later probes, settled payloads,
 keys outside the tables, counts, result layouts and groups in shared memory and L2, segment
 lists, columns that are not 16-byte aligned — against the oracle."""
+import itertools
+
 import numpy as np
 import pytest
 import torch
@@ -118,6 +120,14 @@ def test_probe_and_filter_counts(probes, filters, layout):
         probes = [(*p[:4], 0, -1) for p in probes]
     for after in (-1, 0, len(filters)):
         _check(90_001, probes, 11, filters, res_layout=layout, count_after=after, wild=0.003)
+
+
+@pytest.mark.parametrize("order", list(itertools.permutations(range(4))))
+def test_settled_probes_wherever_they_stand(order):
+    """Two probes settled by their bitmap (one with a group term), one read for its payload, one
+    without a bitmap, in every order."""
+    probes = [(KEY, 3_000, 0, 0.6, 3, -1), D_, (VO, 500, 0, 0.7, 0, -1), C_]
+    _check(100_003, [probes[i] for i in order], 3, wild=0.002, res_layout=L.MB_RES_ENGINE6, total=175)
 
 
 @pytest.mark.parametrize("total,group_mode", [(175, 0), (175, 2), (2_048, 0), (2_049, 0), (9_000, 0)])
