@@ -40,8 +40,9 @@ struct SelPlan {
   long long start_offset;
   int seg_shift;
   unsigned int* status;
-  // sliced kernel: whether the columns read ahead allow 16-byte loads, and the words of the
-  // first probe's presence bitmap (0: none)
+  // sliced kernel: rows a slice, whether the columns read ahead allow 16-byte loads, and the
+  // words of the first probe's presence bitmap (0: none)
+  int slice_rows;
   int vec;
   int bm_words;
 };
@@ -51,7 +52,7 @@ __device__ __forceinline__ bool sel_pass(int x, int mode, int c1, int c2) {
 }
 
 // ---- contiguous rows: slices of 512 ------------------------------------------------------
-// A warp takes slices of 512 consecutive rows, 16 a lane. The columns every row needs — the
+// A warp takes slices of 512 consecutive rows, 16 a lane (of 64 to 256 in short calls). The columns every row needs — the
 // filters, and the first probe's key where its table is small enough for a presence bitmap
 // in shared memory (derived once per CTA) — arrive by bulk copies into the warp's own buffer,
 // and so does the key of the first probe after those while at least one row in 16 of the
@@ -71,7 +72,7 @@ __device__ __forceinline__ bool sel_pass(int x, int mode, int c1, int c2) {
 // instructions a row, 448 us.
 constexpr int kSelMaxWarps = 32;          // one CTA an SM: the bitmap is derived once an SM
 constexpr int kSelItems = 16;             // rows a lane
-constexpr int kSelRows = 32 * kSelItems;  // rows per slice
+constexpr int kSelRows = 32 * kSelItems;  // rows per slice, at most
 constexpr int kSelRound = 64;             // survivors probed at a time (two a lane)
 constexpr int kSelQueue = 2 * kSelRound;  // rows a warp's output queue holds
 constexpr int kSelBitmapMaxSlots = 65536;
@@ -152,7 +153,8 @@ __global__ void __launch_bounds__(kSelMaxWarps * 32, 1) select_slices_kernel(con
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   W& w = reinterpret_cast<W*>(smem)[warp];
   uint32_t* bm = reinterpret_cast<uint32_t*>(smem + nwarps * sizeof(W));
-  const long long nslices = (P.n + kSelRows - 1) / kSelRows;
+  const int rows = P.slice_rows;
+  const long long nslices = (P.n + rows - 1) / rows;
   // consecutive slices per CTA (its warps interleaved): a warp changes segment rarely
   const long long per = (nslices + gridDim.x - 1) / gridDim.x;
   const long long s_end = min(nslices, (blockIdx.x + 1) * per);
@@ -167,7 +169,7 @@ __global__ void __launch_bounds__(kSelMaxWarps * 32, 1) select_slices_kernel(con
 
   // Locate slice s and start its copies (or, where they do not apply, load it).
   auto start = [&](long long s) {
-    const long long r0 = s * kSelRows;
+    const long long r0 = s * rows;
     const bool list = P.seg_group != nullptr;
     const long long v0 = list ? r0 : P.start_offset + r0;
     const long long vseg = P.gpu_cache == nullptr ? 0 : v0 >> P.seg_shift;
@@ -185,17 +187,17 @@ __global__ void __launch_bounds__(kSelMaxWarps * 32, 1) select_slices_kernel(con
     phys0 = P.gpu_cache == nullptr ? v0 : (tab_seg << P.seg_shift) + idx0;
     __syncwarp();
     if (NC == 0) return;
-    in_flight = P.vec && r0 + kSelRows <= P.n && (ND > 0 || staged);
+    in_flight = P.vec && r0 + rows <= P.n && (ND > 0 || staged);
     if (in_flight) {
       if (lane == 0) {
         fence_proxy_async_smem();
-        mbar_arrive_expect_tx(&w.bar, (staged ? NC : ND) * kSelRows * 4);
+        mbar_arrive_expect_tx(&w.bar, (staged ? NC : ND) * rows * 4);
 #pragma unroll
         for (int c = 0; c < NC; ++c)
-          if (c < ND || staged) bulk_g2s(w.stage[c], w.col[tab][c] + idx0, kSelRows * 4, &w.bar, policy);
+          if (c < ND || staged) bulk_g2s(w.stage[c], w.col[tab][c] + idx0, rows * 4, &w.bar, policy);
       }
     } else {
-      const int have = static_cast<int>(min(static_cast<long long>(kSelRows), P.n - r0));
+      const int have = static_cast<int>(min(static_cast<long long>(rows), P.n - r0));
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
         const int* col = w.col[tab][c] + idx0;
@@ -255,7 +257,7 @@ __global__ void __launch_bounds__(kSelMaxWarps * 32, 1) select_slices_kernel(con
     const long long phys = phys0, idx = idx0;
     const bool staged_now = staged;
     const int* const* cols = w.col[tab];
-    const int have = static_cast<int>(min(static_cast<long long>(kSelRows), P.n - s * kSelRows));
+    const int have = static_cast<int>(min(static_cast<long long>(rows), P.n - s * rows));
     if (NC > 0 && in_flight) {
       const bool ok = mbar_wait_bounded(&w.bar, parity);
       parity ^= 1u;
@@ -333,7 +335,7 @@ __global__ void __launch_bounds__(kSelMaxWarps * 32, 1) select_slices_kernel(con
       if (lane >= o) incl += y;
     }
     const int cnt = __shfl_sync(0xffffffffu, incl, 31);
-    staged = cnt >= kSelRows / 16;
+    staged = cnt >= rows / 16;
     uint16_t* at = w.off + (incl - own);
     while (sel) {
       const int i = __ffs(sel) - 1;
@@ -539,12 +541,13 @@ int select_init_device(const DeviceState& ds) {
 }
 
 static int launch_slices(SelPlan& P, const DeviceState& ds, cudaStream_t st) {
-  // The first probe goes to a bitmap when its table is small and not read for a handful of
-  // rows: every CTA reads the whole table once, to save a scattered load (a cycle of the SM's
-  // load path and an L2 trip) per row. A 40,000-slot table of 8-byte slots, select and two
-  // probes: 300,000 rows 16.3 against 18.8 us, 24,000,000 rows 82.6 against 222.1 us; 2,000
-  // slots: 9.1 against 19.1 and 73.6 against 203.7 us.
-  const bool bm = P.np > 0 && P.pslots[0] <= kSelBitmapMaxSlots && P.n / 4 >= P.pslots[0];
+  // The first probe goes to a bitmap when its table is small and enough rows are to be read:
+  // every CTA reads the whole table once, to save a scattered load (a cycle of the SM's load path
+  // and an L2 trip) per row. A 40,000-slot table of 8-byte slots, a filter and a second probe:
+  // 24,000,000 rows 96 against 376 us. Its cost shows below some 32 rows a slot: 800,000 rows, each
+  // probe keeping 5, 20, 50 and 100 %, 21, 22, 26 and 34 us with it and 17, 18, 19 and 24 without;
+  // 1,300,000 rows 20, 22, 28 and 42 against 22, 25, 26 and 36.
+  const bool bm = P.np > 0 && P.pslots[0] <= kSelBitmapMaxSlots && P.n / 32 >= P.pslots[0];
   const bool key = P.np > (bm ? 1 : 0);
   const int nc = P.nf + (bm ? 1 : 0) + (key ? 1 : 0);
   P.bm_words = bm ? P.pslots[0] / 32 + 1 : 0;  // slots 0 .. pslots (the last one absent)
@@ -555,15 +558,18 @@ static int launch_slices(SelPlan& P, const DeviceState& ds, cudaStream_t st) {
     for (int f = 0; f < P.nf; ++f) P.vec = P.vec && aligned16(P.fcol[f]);
     for (int p = 0; p < P.np && p < nc - P.nf; ++p) P.vec = P.vec && aligned16(P.pkey[p]);
   }
-  // as many warps as their buffers leave room for; short calls spread over the SMs, a few
-  // slices each
-  const long long nslices = (P.n + kSelRows - 1) / kSelRows;
-  long long blocks = (nslices + 3) / 4;
-  if (blocks > ds.num_sms) blocks = ds.num_sms;
-  const long long per = (nslices + blocks - 1) / blocks;
+  // as many warps as their buffers leave room for
   int warps = (ds.max_smem_optin - 4 * P.bm_words) / warp_bytes(nc);
   if (warps > kSelMaxWarps) warps = kSelMaxWarps;
-  if (warps > per && per >= 16) warps = static_cast<int>(per);
+  // Smaller slices while every one of them still has a warp of its own: a slice's rounds run one
+  // after the other. 300,000 rows (the call above, no bitmap, all rows kept) 14.3 us, 500,000 18; 24
+  // and 30 with the bitmap, 36 with slices of 512 as well; one row a lane 17 and 23.
+  P.slice_rows = kSelRows;
+  const long long at_once = static_cast<long long>(warps) * ds.num_sms;
+  while (P.slice_rows > 64 && (P.n + P.slice_rows / 2 - 1) / (P.slice_rows / 2) <= at_once) P.slice_rows /= 2;
+  const long long nslices = (P.n + P.slice_rows - 1) / P.slice_rows;
+  long long blocks = (nslices + 3) / 4;
+  if (blocks > ds.num_sms) blocks = ds.num_sms;
   const int smem = warps * warp_bytes(nc) + 4 * P.bm_words;
   if (launch_dependent(kSlices[P.nf][2 * (bm ? 1 : 0) + (key ? 1 : 0)], static_cast<int>(blocks), warps * 32,
                        static_cast<size_t>(smem), st, P) != cudaSuccess)

@@ -131,3 +131,41 @@ def test_segments(size, order):
 
 def test_full_list():
     _check(200_001, [], [(L.MB_HT_VAL_OFF, 500, 0, 0.9)], 9, capacity=1_000)
+
+
+# one filter and two probes, the first decided by its bitmap: 23 warps an SM
+@pytest.mark.parametrize("rows,slices", [(64, 23), (128, 23), (256, 23), (512, 23), (512, 60)])
+@pytest.mark.parametrize("more", [-1, 0, 1, 129])
+def test_slice_sizes(rows, slices, more):
+    """Calls around the most rows that slices of a size take, and of more than a slice a warp."""
+    _check(rows * slices * 148 + more, [(BETWEEN, 3, 16)],
+           [(LAYOUTS[2], 100, 0, 0.5), (LAYOUTS[1], 5_000, 0, 0.4)], rows + more)
+
+
+@pytest.mark.parametrize("first", LAYOUTS)
+@pytest.mark.parametrize("second", [None, *LAYOUTS])
+@pytest.mark.parametrize("filters", [[], [(BETWEEN, 1, 18), (BETWEEN, 0, 19), (BETWEEN, 2, 19)]])
+def test_layouts_decided_by_a_bitmap(first, second, filters):
+    """The first table's bitmap from 32 rows a slot on, the second's table read."""
+    probes = [(first, 3_001, 0, 0.3)] + ([(second, 70_001, 5, 0.6), (second, 63, -7, 0.9)] if second is not None else [])
+    for n in (32 * 3_001 - 1, 32 * 3_001, 700_003):
+        _check(n, filters, probes, 7, wild=0.01)
+
+
+@pytest.mark.parametrize("slots", [33, 65_535, 65_536, 65_537])
+@pytest.mark.parametrize("layout", LAYOUTS)
+def test_largest_bitmaps(slots, layout):
+    _check(32 * 65_537 + 11, [], [(layout, slots, 19, 0.2), (L.MB_HT_KEY, 1_000, 0, 0.5)], slots, wild=0.001)
+
+
+@pytest.mark.parametrize("share", [0.0, 0.002, 1.0])
+def test_rows_dropped_before_the_last_probe(share):
+    """Rounds of which no row, hardly a row and every row goes on to the second and third probe."""
+    _check(300_007, [], [(L.MB_HT_VAL_OFF, 66_000, 0, share), (L.MB_HT_KEY, 500, 0, 0.5), (L.MB_HT_KEY_VAL, 66_000, 0, 0.9)],
+           5, wild=0.001)
+
+
+@pytest.mark.parametrize("size,order", [(512, [5, 2, 0, 1]), (1 << 16, [6, 1, 0, 4, 3])])
+def test_segments_with_a_bitmap(size, order):
+    _check(len(order) * size - 77, [(BETWEEN, 2, 15)], [(L.MB_HT_VAL_OFF, 60, 0, 0.5), (L.MB_HT_KEY_VAL, 900, 0, 0.7)],
+           size, segment=(size, order))
