@@ -416,8 +416,9 @@ typedef struct mb_batch_args {
   void* workspace;                        /* device, >= mb_batch_workspace_bytes(), 16-byte aligned */
   size_t workspace_bytes;
   /* consumer threads x rows per thread per stage: 256x4, 512x4, 512x2, 768x1, 768x2 or
-   * 960x1 (both 0 = 768x2 for up to 64 queries, else 960x1, or 768x1 where shared memory
-   * does not hold these; one of them 0 = 768 threads or 1 row); stages 2..8 (0 = 2); grid 0 = one CTA per SM */
+   * 960x1 (both 0 = 768x2 for up to 64 queries, else 960x1, or 768x1 for few rows and where
+   * shared memory does not hold these; one of them 0 = 768 threads or 1 row); stages 2..8
+   * (0 = 2); grid 0 = one CTA per SM */
   int threads, items_per_thread, stages, grid;
   int smem_group_bytes;                   /* shared memory for small group arrays; -1 default, 0 none */
   /* Segment-cache addressing (optional; src/gpudb/GPUProcessing.h:54-67 for one query):

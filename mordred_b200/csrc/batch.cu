@@ -1308,13 +1308,16 @@ extern "C" int mb_batch_run(const mb_batch_args* a, mb_stream_t stream) {
 
   // Defaults: up to 64 queries a row has few matches and the work per row decides, so a lane
   // takes two rows at a time (24 queries over 75 M rows: 768x2 1.76 ms, 960x1 2.22, 768x1
-  // 2.52); above, the match lists are full anyway and one more warp a scheduler hides more
+  // 2.52) unless an SM gets one tile at most, which half the rows finish sooner (24 queries over
+  // 113,000 rows: 768x1 36 us, 768x2 40; over 150,000: 42 and 40; over less than a tile's 1,536 rows,
+  // read without the ring, 37 and 31); above, the match lists are full anyway and one more warp a scheduler hides more
   // (120 queries over 20 M rows: 960x1 1.10 ms, 768x1 1.20, 768x2 1.33; 256 queries, with
   // group arrays filling the shared memory: 2.21, 2.30, 2.21). A call that sets one of the
   // two gets 768 threads or one row for the other.
   const bool by_size = a->threads == 0 && a->items_per_thread == 0;
   int threads = a->threads ? a->threads : by_size && P.nwords > 2 ? 960 : 768;
-  int items = a->items_per_thread ? a->items_per_thread : by_size && P.nwords <= 2 ? 2 : 1;
+  const bool one_tile = P.n >= 2 * 768 && P.n <= 768ll * ds->num_sms;
+  int items = a->items_per_thread ? a->items_per_thread : by_size && P.nwords <= 2 && !one_tile ? 2 : 1;
   auto variant = [&]() -> const BatchVariant* {
     for (const BatchVariant& v : kBatchVariants)
       if (v.warps * 32 == threads && v.items == items && v.nwm == P.nwords) return &v;

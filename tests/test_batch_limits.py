@@ -71,3 +71,10 @@ def test_more_tables_than_shared_memory_holds(count, values, launch):
         queries.append(dict(layout=layout, keys=keys, op=op, agg=[B.FACT[a] for a in agg], total=130, dims=i % 16,
                             preds=preds))
     _check(6_401, queries, count + values, **launch)
+
+
+@pytest.mark.parametrize("n", [1_535, 1_536, 1_537, 768 * 148, 768 * 148 + 1, 1_536 * 148 + 5])
+@pytest.mark.parametrize("count", [24, 64])
+def test_default_launches_of_few_rows(n, count):
+    """Up to a tile of 768 rows an SM, and more."""
+    M._check(n, M._queries(count, n, 3), n)
