@@ -262,11 +262,16 @@ int launch_star(const mb_star_args* a, cudaStream_t stream, int count32, const D
   }
 
   // ---- calls with probes and no launch shape of their own -------------------------
-  // The ring kernel is the faster one at every size measured against the tile kernels' tuned
-  // shapes (Query B over 1,000,000 rows 16 against 24 us, 120,000,000 rows 341 against 614;
-  // Query A 350 against 457; the engine's group-by over 23 segments 103 against 159). The tile
-  // kernels keep what it does not take: calls without a probe (every column of every row is
-  // needed; the tiles stream at the copy rate), columns that bulk copies cannot start on,
+  // The ring kernel is the faster one against the tile kernels' tuned shapes, whatever share of
+  // the rows the probes keep (which the host does not know): Query B over 1,000,000 rows 16 against
+  // 24 us, 120,000,000 rows 341 against 614; Query A 350 against 457; the engine's group-by over 23
+  // segments 103 against 159. 24,000,000 rows, every probe keeping 5, 20, 50 and 100 % of what
+  // reaches it: one probe 69, 112, 185 and 275 us against 130, 195, 375 and 652; four probes 58, 77,
+  // 179 and 409 against 110, 135, 280 and 560; a filter and three probes, from 20 % on, 106, 206 and
+  // 431 against 161, 253 and 439. With every row kept it was slower in two shapes: sums in L2
+  // (below), and two bitmap tables whose payloads are read again before a third (604 against 581).
+  // The tile kernels keep what it does not take: calls without a probe (every column of every
+  // row is needed; the tiles stream at the copy rate), columns that bulk copies cannot start on,
   // payload factors, 2^32 rows and more, and calls that ask for a launch shape.
   if (a->mirrors < 0 || a->mirrors > 2) return MB_ERR_ARG;
   if (a->pack < 0 || a->pack > 4) return MB_ERR_ARG;
@@ -278,6 +283,11 @@ int launch_star(const mb_star_args* a, cudaStream_t stream, int count32, const D
   if (P.np > 0 && a->agg_op != MB_AGG_MUL_PAYLOAD && tiles && P.n < (1ll << 32) &&
       (P.gpu_cache == nullptr || (1 << P.seg_shift) >= tile_of_defaults) && a->threads == 0 &&
       a->items_per_thread == 0 && a->stages == 0 && a->grid == 0 && a->mirrors != 2 && a->pack == 0 && a->group_mode != 1) {
+    // More than 2,048 groups stay in L2: the flush of every CTA's array, and the L1 it takes, cost
+    // more than the atomics save while the probes keep few rows. Three probes over 24,000,000 rows,
+    // each keeping 20, 50 and 100 %: 2,100 groups 76, 149 and 633 us against 77, 146 and 316 in shared
+    // memory (the tile kernels, in L2: 117, 202 and 604), 4,200 groups 76, 147 and 545 against 102, 214
+    // and 441 (513); over 300,000 rows, all of 2,100 to 3,200 groups, 10.5 against 11.1 at 20 %.
     const int big = P.res_layout != MB_RES_SCALAR && P.total_val > 2048 ? 2 : 0;
     const int e = launch_ring(P, a->group_mode ? a->group_mode : big, *ds, stream);
     if (e != MB_ERR_SIZE) return e;

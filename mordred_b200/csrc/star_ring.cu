@@ -537,11 +537,14 @@ int ring_init_device(const DeviceState& ds) {
 }
 
 int launch_ring(StarPlan& P, int group_mode, const DeviceState& ds, cudaStream_t stream) {
-  // leading probes decided by a bitmap: given by the caller, or derived by every CTA from a
-  // table it reads whole — a small one, and not for a handful of rows. A call with the first
-  // probe (40,000 slots) derived against looked up in L2 row by row: Query A over 120,000,000
-  // rows 361 against 865 us, Query B 375 and 954, over 1,000,000 rows 31 and 42; the engine's
-  // group-by (8-byte slots) over 23 segments 137 and 238.
+  // Leading probes decided by a bitmap: given by the caller, or derived by every CTA from a table
+  // it reads whole — a small one, and not for a handful of rows. A call with the first probe
+  // (40,000 slots) derived against looked up in L2 row by row: Query A over 120,000,000 rows 361
+  // against 865 us, Query B 375 and 954; the engine's group-by (8-byte slots) over 23 segments 137
+  // and 238. Key tables gain at every size measured, down to 2 rows a slot (four probes, 80,000
+  // rows: 11.2 and 13.5 us), tables of 8-byte slots up to 20,000 slots likewise (three probes that
+  // keep 20 %, 160,000 rows, 20,000 slots: 10.8 and 12.5), 40,000 of them from some 32 rows a slot
+  // on (1,000,000 rows 15.3 and 14.0, 1,300,000 rows 18.4 and 21.4).
   P.n_dense = P.sparse_p0 = 0;
   P.dense_bias = 0;
   int off = 0;
@@ -561,7 +564,8 @@ int launch_ring(StarPlan& P, int group_mode, const DeviceState& ds, cudaStream_t
     if (P.n_dense < p) continue;
     const int bytes = (P.p_slots[p] / 32 + 1) * 4;  // slots 0 .. p_slots (the last one absent)
     const int derive_max = P.p_layout[p] == MB_HT_KEY ? 8 * kBitmapSmemMaxBytes : kBitmapDeriveMaxSlots8;
-    const bool have = P.p_presence[p] != nullptr || (P.p_slots[p] <= derive_max && P.n / 4 >= P.p_slots[p]);
+    const int rows_a_slot = P.p_layout[p] == MB_HT_KEY || P.p_slots[p] <= 20'000 ? 4 : 32;
+    const bool have = P.p_presence[p] != nullptr || (P.p_slots[p] <= derive_max && P.n / rows_a_slot >= P.p_slots[p]);
     if (!have || bytes > kBitmapSmemMaxBytes + 4 || bm_total + bytes > kBitmapSmemTotalBytes) continue;
     P.p_bm_off[p] = off + bm_total;
     P.p_bm_words[p] = bytes / 4;
@@ -598,8 +602,9 @@ int launch_ring(StarPlan& P, int group_mode, const DeviceState& ds, cudaStream_t
   for (int f = 0; f < P.nf; ++f) P.r_fcol[f] = staged(P.f_col[f]);
   for (int p = 0; p < P.n_dense; ++p) P.r_pcol[p] = staged(P.p_col[p]);
   P.r_kcol = key ? staged(P.p_col[P.sp_ord[0]]) : 0;
-  // one CTA an SM with as many warps as their buffers leave room for; short calls spread over
-  // the SMs first
+  // one CTA an SM with as many warps as their buffers leave room for (also where fewer
+  // have a slice: they help to derive the bitmaps — as many warps as slices took 13.9 against 11.9 us
+  // for four probes over 600,000 rows); short calls spread over the SMs first
   const int budget = ds.max_smem_optin - 2048 - static_cast<int>(2 * kRingMaxWarps * sizeof(unsigned long long));
   int warps = (budget - off) / ring_warp_bytes(P.r_nst);
   if (warps > kRingMaxWarps) warps = kRingMaxWarps;
@@ -607,8 +612,6 @@ int launch_ring(StarPlan& P, int group_mode, const DeviceState& ds, cudaStream_t
   const long long nslices = (P.n + kRingRows - 1) / kRingRows;
   long long blocks = (nslices + 3) / 4;
   if (blocks > ds.num_sms) blocks = ds.num_sms;
-  const long long per = (nslices + blocks - 1) / blocks;
-  if (warps > per && per >= 16) warps = static_cast<int>(per);
   P.smem_total = off + warps * ring_warp_bytes(P.r_nst);
   const KernelFn fn = kRing[P.nf > 0 ? 1 : 0][P.n_dense > 1 ? 2 : P.n_dense][key ? 1 : 0];
   if (launch_dependent(fn, static_cast<int>(blocks), warps * 32, static_cast<size_t>(P.smem_total), stream, P) !=

@@ -149,6 +149,14 @@ def test_bitmap_sizes(slots, layout, presence):
     _check(1_100_003, [(layout, slots, 2, 0.3, 0, -1), (KV, 500, 0, 0.6, 1, 0)], slots, wild=0.001, presence=presence)
 
 
+@pytest.mark.parametrize("slots,n", [(20_000, 80_000), (20_000, 79_999), (20_001, 640_032), (20_001, 640_031),
+                                     (65_536, 2_097_152), (65_536, 2_097_151)])
+@pytest.mark.parametrize("layout", [KV, VO])
+def test_rows_from_which_a_bitmap_is_derived(slots, n, layout):
+    """Tables of 8-byte slots: 4 rows a slot, above 20,000 slots 32."""
+    _check(n, [(layout, slots, 2, 0.3, 7, 1), (KEY, 500, 0, 0.6, 0, -1)], slots, wild=0.001, res_layout=L.MB_RES_ENGINE6)
+
+
 @pytest.mark.parametrize("size,order", [(2048, [3, 0, 5, 1]), (4096, [6, 1, 0, 4, 3])])
 def test_segments(size, order):
     _check(len(order) * size - 5, [S_, C_, P_, D_], size, [(BETWEEN, 1, 18)], segment=(size, order))
