@@ -125,7 +125,9 @@ typedef struct mb_star_args {
   const short* segment_group; /* virtual segment -> segment id; NULL: (start_offset + r) / segment_size */
   int64_t start_offset;
   int segment_size;           /* power of two (reference: 1,048,576) */
-  /* launch configuration; 0 = the tuned default for this shape */
+  /* Launch configuration of the tile-staged kernels; 0 = the tuned default for this shape. Calls
+   * with a probe over aligned columns that set none of threads, items_per_thread, stages, grid
+   * and pack (nor mirrors 2, nor group_mode 1) run a kernel without these choices. */
   int threads;                /* consumer threads per CTA: 128, 256 or 512 (plus one producer warp);
                                * 640 or 768 (20 or 24 warps sharing 16 tile slices, 8 rows a
                                * thread) where the query shape has such a variant, else 512 */
@@ -440,8 +442,9 @@ int mb_pat_build(const int* dim_key, int num_rows, int key_min, int slots,
                  const int* attr0, int field0, const int* attr1, int field1,
                  const int* attr2, int field2, unsigned int* words, mb_stream_t stream);
 
-/* Device workspace the batch needs: for every predicate attribute, a table mapping each
- * value of the queries' range hull to the bitmask of queries that accept it. */
+/* Device workspace the batch needs: tables mapping each value of the queries' range hull on a
+ * predicate attribute — or each combination of values of several small attributes — to the
+ * bitmask of queries that accept it. */
 size_t mb_batch_workspace_bytes(const mb_batch_args* args);
 
 /* Run a batch of queries: one small kernel fills the workspace's query masks, then one

@@ -1,4 +1,7 @@
-"""Autotuner for the fused star kernel.
+"""Autotuner for the tile-staged star kernels: what filter-aggregates run, and calls that the
+default kernel of star queries with probes (``csrc/star_ring.cu``, which has no launch shape to
+tune) does not take — misaligned columns, payload factors, a launch shape of their own. Every
+configuration tried here sets a launch shape, so the probe shapes are those kernels' too.
 
 For each query shape of the workload (the filter-aggregate, Query A, Query B and the
 engine's four-table group-by) it times every launch configuration — consumer threads

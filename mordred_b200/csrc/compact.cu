@@ -7,9 +7,10 @@
 // cross PCIe as offset lists (src/gpudb/CPUGPUProcessing.cu:60-144 switch_device_fact).
 // Restates the reference's compaction kernels filter_GPU2/3, filter_probe_GPU2/3 and
 // probe_GPU2/3 (src/gpudb/GPUProcessing.h:496-925, 1174-1383), which scan per block and
-// take one atomicAdd on the output cursor per block; here each warp ballots its 32 rows
-// and takes one atomicAdd per warp, so the list order is not deterministic (it never is
-// in the reference either) while its set of rows is.
+// take one atomicAdd on the output cursor per block; here a warp takes one for each 64 rows it
+// has queued (contiguous rows) or for the survivors among 32 rows (listed rows, small segments),
+// so the list order is not deterministic (it never is in the reference either) while its set of
+// rows is.
 //
 // Probe outputs per layout: MB_HT_VAL_OFF (engine builds) — present when the row word
 // ht[2h+1] != 0, output ht[2h+1] - 1, the dimension row (BlockLibrary.cuh:9-33);

@@ -1,7 +1,8 @@
-// star.cuh — the fused star-query pipeline: its device-side plan and the host launcher.
-//
-// One persistent, warp-specialised kernel runs filter -> chained perfect-hash probes ->
-// group-by / aggregate over the fact table:
+// star.cuh — the fused star-query pipeline (filter -> chained perfect-hash probes -> group-by /
+// aggregate over the fact table): its device-side plan and the host launcher. Calls with a probe
+// run star_ring.cu's kernel by default. The tile-staged kernels (star_impl.cuh), which keep
+// filter-aggregates, columns bulk copies cannot start on, payload factors and calls with a
+// launch shape of their own, are persistent and warp-specialised:
 //   * a producer warp streams fact-column tiles into shared memory with 1-D bulk copies
 //     (cp.async.bulk, no multicast) into a ring of stages, each guarded by a "full"
 //     mbarrier (transaction bytes) and an "empty" mbarrier (one arrival per consumer warp);
